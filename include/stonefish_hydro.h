@@ -865,11 +865,13 @@ typedef struct hydro_nn_net {
  * rows [rows[s], rows[s] + batch) of the bf16 network inputs X [n_rows][k_0]
  * and of the FP32 targets T [n_rows][n_out], runs the forward and backward
  * passes and updates every layer with learning rate lr[s] and step count
- * step0 + s + 1 (rows and lr are host arrays of n_steps).  It launches the
- * kernels of hydro_nn_gemm, hydro_nn_mse_grad, hydro_nn_transpose,
- * hydro_nn_colsum and hydro_nn_adamw with the same arguments in the same
- * order as calling those one by one, so the trained weights are the same
- * bits; a step then costs no round trip through the caller. */
+ * step0 + s + 1 (rows and lr are host arrays of n_steps).  The products and
+ * sums run in the order of hydro_nn_gemm, hydro_nn_mse_grad,
+ * hydro_nn_transpose, hydro_nn_colsum and hydro_nn_adamw, so the trained
+ * weights are the same bits as calling those one by one; a step costs no
+ * round trip through the caller, and a 64-256-256-256-64 network runs it in
+ * three fused launches.  w, b, their moments and bf16 copies, gw, gb and
+ * *loss are the results; z, x, dz and xt are scratch. */
 hydro_status hydro_nn_train(hydro_ctx* ctx, const hydro_nn_net* net, const void* X, const float* T,
                             int64_t n_rows, const int64_t* rows, const float* lr, int32_t n_steps,
                             int32_t step0, float beta1, float beta2, float eps, float weight_decay,

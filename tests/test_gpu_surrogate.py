@@ -370,6 +370,29 @@ def test_native_training_loop_matches_step_by_step_calls(hctx):
     assert torch.equal(a.layers[0]["w"], b.layers[0]["w"])
 
 
+@pytest.mark.parametrize("batch", [64, 320, 2112, 4096])
+def test_fused_training_step_matches_step_by_step_calls(hctx, batch):
+    """The fused step (rows, gradients, update) against the single entry
+    points where its splits can go wrong: one 64-row tile, one slice, column
+    slabs that do not divide the batch, and the full split; weights, gradients
+    and moments are the same bits."""
+    rng = np.random.default_rng(batch)
+    n = 2 * batch + 5
+    feats = _dev(rng.normal(size=(n, S.N_FEAT)))
+    targ = _dev(rng.normal(size=(n, S.N_OUT)) * 40.0 + 5.0)
+    nets, losses = [], []
+    for native in (True, False):
+        sur = S.Surrogate(hctx, hidden=256, seed=5, batch=batch)
+        sur.fit_normalisation(feats, targ)
+        losses.append(sur.fit(feats, targ, epochs=2, lr=3e-3, warmup=2, native=native)["loss"])
+        nets.append(sur)
+    torch.cuda.synchronize()
+    np.testing.assert_allclose(losses[0], losses[1], rtol=1e-12)
+    for La, Lb in zip(nets[0].layers, nets[1].layers):
+        for f in ("w", "b", "gw", "gb", "mw", "vw", "mb", "vb", "w16", "wt16"):
+            assert torch.equal(La[f], Lb[f]), f
+
+
 @pytest.mark.parametrize("n", [1000, 4096])
 def test_fused_tensor_core_inference_matches_gemm_path(hctx, n):
     """hydro_nn_mlp_tc (tcgen05, one kernel) against the four mma.sync GEMMs:
