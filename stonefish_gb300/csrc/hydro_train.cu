@@ -5,7 +5,7 @@
 // Step by step the layers' products, epilogues, transposes, column sums and
 // parameter updates are 36 launches of 3 to 15 us whose operands travel
 // through memory between them: 228 us at batch 4096, of which the tensor
-// cores need about 3; the fused step takes 52 us.  Here
+// cores need about 3; the fused step takes 47 us.  Here
 //   1. train_rows_kernel: 32 rows of the batch go through the four layers,
 //      the loss gradient and back to the first layer's pre-activations in
 //      one CTA.  No row needs another one, so the activations stay in shared
@@ -36,11 +36,14 @@ namespace train {
 constexpr int kRows = 32;        // batch rows per CTA of the row kernel
 constexpr int kH = 256;
 constexpr int kLdA = kH + 8;     // activation row stride in shared memory (an odd number of 16-byte units)
-constexpr int kThreads = 256;    // eight warps, each 32 rows x 32 columns
+// Sixteen warps, each 32 rows x 16 columns: with eight warps of 32 x 32 the
+// kernel issued an instruction in 23% of its cycles (two warps per scheduler
+// waiting on mma and ldmatrix results) and took 29 us; with sixteen 22 us.
+constexpr int kThreads = 512;
 constexpr int kStages = 3;
 constexpr int kStageBytes = 64 * kH * 2;   // 64 weight rows
 constexpr int kChunks = 22;      // weight chunks of the seven products
-constexpr size_t kRowsSmem = (size_t)kStages * kStageBytes + 2 * kRows * kLdA * 2;
+constexpr size_t kRowsSmem = (size_t)kStages * kStageBytes + 2 * kRows * kLdA * 2 + (3 * kH + 64) * 4;
 
 __device__ __forceinline__ void cp16(void* dst, const void* src)
 {
@@ -50,6 +53,12 @@ __device__ __forceinline__ void cp16(void* dst, const void* src)
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+
+// Programmatic dependent launch: the step's kernels are a chain, and each is
+// launched while the one before it runs, so that its CTAs are there when the
+// last one of that ends.  Nothing is read or written before dependency_wait().
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Chunk i of the weights in the order the row kernel multiplies by them:
 // 64 rows of the layers' weights going forward, of their transposes going
@@ -70,13 +79,13 @@ __device__ __forceinline__ void load_weights(const RowsParams& P, unsigned char*
         unsigned char* st = smem + (i % kStages) * kStageBytes;
         if (narrow) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
+            for (int j = 0; j < 64 * 8 / kThreads; ++j) {
                 const int u = threadIdx.x + j * kThreads, r = u >> 3, c = u & 7;
                 cp16(st + r * 128 + ((c ^ (r & 7)) << 4), src + r * 64 + c * 8);
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 64 * 32 / kThreads; ++j) {
                 const int u = threadIdx.x + j * kThreads, r = u >> 5, c = u & 31;
                 cp16(st + r * 512 + ((c ^ (r & 7)) << 4), src + r * kH + c * 8);
             }
@@ -96,17 +105,20 @@ __device__ __forceinline__ void store_rows(const bf16* buf, bf16* dst, int cols)
     }
 }
 
-// One product of the row kernel: N = 256, warp w's 32 x 32 tile at column
-// 32 w.  A (32 x 64 n_chunks) is in `buf`, whose contents also go to `out`
+// One warp's 32 x 16 accumulators of a 256-column product.
+typedef float Tile[2][2][4];
+
+// One product of the row kernel: N = 256, warp w's 32 x 16 tile at column
+// 16 w.  A (32 x 64 n_chunks) is in `buf`, whose contents also go to `out`
 // once they are visible; the weights arrive as chunks first, first + 1, ...
 __device__ __forceinline__ void product256(const RowsParams& P, unsigned char* smem, const bf16* buf, int first,
-                                           int n_chunks, bf16* out, int out_cols, float (&acc)[2][4][4])
+                                           int n_chunks, bf16* out, int out_cols, Tile& acc)
 {
-    const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) * 32;
+    const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) * 16;
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
 #pragma unroll 1
@@ -119,70 +131,60 @@ __device__ __forceinline__ void product256(const RowsParams& P, unsigned char* s
         const unsigned char* st = smem + (i % kStages) * kStageBytes;
 #pragma unroll
         for (int kk = 0; kk < 64; kk += 16) {
-            uint32_t a[2][4], b[4][2];
+            uint32_t a[2][4], t[4];
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi)
                 ldsm_x4(a[mi], buf + (mi * 16 + (lane & 15)) * kLdA + q * 64 + kk + (lane >> 4) * 8);
+            const int j = lane >> 3, r = kk + (lane & 7) + 8 * (j & 1), c = (wn >> 3) + (j >> 1);
+            ldsm_x4_t(t, st + r * 512 + ((c ^ (r & 7)) << 4));
 #pragma unroll
-            for (int nj = 0; nj < 2; ++nj) {
-                const int j = lane >> 3, r = kk + (lane & 7) + 8 * (j & 1), c = (wn >> 3) + nj * 2 + (j >> 1);
-                uint32_t t[4];
-                ldsm_x4_t(t, st + r * 512 + ((c ^ (r & 7)) << 4));
-                b[2 * nj][0] = t[0];
-                b[2 * nj][1] = t[1];
-                b[2 * nj + 1][0] = t[2];
-                b[2 * nj + 1][1] = t[3];
+            for (int mi = 0; mi < 2; ++mi) {
+                mma_bf16(acc[mi][0], a[mi], t[0], t[1]);
+                mma_bf16(acc[mi][1], a[mi], t[2], t[3]);
             }
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) mma_bf16(acc[mi][ni], a[mi], b[ni][0], b[ni][1]);
         }
     }
 }
 
-// Hidden layer: bias, then SiLU into `y`; acc keeps the pre-activations.
-__device__ __forceinline__ void epilogue_silu(float (&acc)[2][4][4], const float* bias, bf16* y)
+// Hidden layer: z = acc + bias, SiLU(z) into `y`; acc keeps SiLU'(z), all
+// that the way back needs of z (one sigmoid serves both).
+__device__ __forceinline__ void epilogue_silu(Tile& acc, const float* bias, bf16* y)
 {
-    const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) * 32;
+    const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) * 16;
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
+    for (int ni = 0; ni < 2; ++ni) {
         const int c = wn + ni * 8 + (lane & 3) * 2;
-        const float b0 = bias[c], b1 = bias[c + 1];
+        const float2 b = *reinterpret_cast<const float2*>(bias + c);
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = mi * 16 + (lane >> 2) + 8 * h;
-                const float v0 = acc[mi][ni][2 * h] + b0, v1 = acc[mi][ni][2 * h + 1] + b1;
-                acc[mi][ni][2 * h] = v0;
-                acc[mi][ni][2 * h + 1] = v1;
+                const float z0 = acc[mi][ni][2 * h] + b.x, z1 = acc[mi][ni][2 * h + 1] + b.y;
+                const float s0 = sigmoidf_(z0), s1 = sigmoidf_(z1);
                 *reinterpret_cast<__nv_bfloat162*>(y + r * kLdA + c) =
-                    __nv_bfloat162(__float2bfloat16(v0 * sigmoidf_(v0)), __float2bfloat16(v1 * sigmoidf_(v1)));
+                    __nv_bfloat162(__float2bfloat16(z0 * s0), __float2bfloat16(z1 * s1));
+                acc[mi][ni][2 * h] = s0 + z0 * s0 * (1.f - s0);
+                acc[mi][ni][2 * h + 1] = s1 + z1 * s1 * (1.f - s1);
             }
     }
 }
 
-// Gradient through the SiLU of a hidden layer with pre-activations z.
-__device__ __forceinline__ void epilogue_grad(const float (&acc)[2][4][4], const float (&z)[2][4][4], bf16* y)
+// Gradient through a hidden layer's SiLU, d its derivative.
+__device__ __forceinline__ void epilogue_grad(const Tile& acc, const Tile& d, bf16* y)
 {
-    const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) * 32;
+    const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) * 16;
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
-        const int c = wn + ni * 8 + (lane & 3) * 2;
+    for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int r = mi * 16 + (lane >> 2) + 8 * h;
-                const float v0 = acc[mi][ni][2 * h], v1 = acc[mi][ni][2 * h + 1];
-                const float z0 = z[mi][ni][2 * h], z1 = z[mi][ni][2 * h + 1];
-                const float s0 = sigmoidf_(z0), s1 = sigmoidf_(z1);
+                const int r = mi * 16 + (lane >> 2) + 8 * h, c = wn + ni * 8 + (lane & 3) * 2;
                 *reinterpret_cast<__nv_bfloat162*>(y + r * kLdA + c) =
-                    __nv_bfloat162(__float2bfloat16(v0 * (s0 + z0 * s0 * (1.f - s0))),
-                                   __float2bfloat16(v1 * (s1 + z1 * s1 * (1.f - s1))));
+                    __nv_bfloat162(__float2bfloat16(acc[mi][ni][2 * h] * d[mi][ni][2 * h]),
+                                   __float2bfloat16(acc[mi][ni][2 * h + 1] * d[mi][ni][2 * h + 1]));
             }
-    }
 }
 
 }  // namespace train
@@ -193,30 +195,30 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
     extern __shared__ __align__(128) unsigned char smem[];
     bf16* buf0 = reinterpret_cast<bf16*>(smem + kStages * kStageBytes);
     bf16* buf1 = buf0 + kRows * kLdA;
+    float* bias = reinterpret_cast<float*>(buf1 + kRows * kLdA);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t row0 = (size_t)blockIdx.x * kRows;
+    dependency_wait();
+    launch_dependents();
     load_weights(P, smem, 0);
     load_weights(P, smem, 1);
-    {
+    if (tid < 256) {
         const int r = tid >> 3, c = tid & 7;
         *reinterpret_cast<uint4*>(buf0 + r * kLdA + c * 8) =
             *reinterpret_cast<const uint4*>(P.x0 + (row0 + r) * 64 + c * 8);
     }
-    float z0[2][4][4], z1[2][4][4], z2[2][4][4];
-    product256(P, smem, buf0, 0, 1, nullptr, 0, z0);
-    epilogue_silu(z0, P.bias[0], buf1);
-    product256(P, smem, buf1, 1, 4, P.x[0] + row0 * kH, kH, z1);
-    epilogue_silu(z1, P.bias[1], buf0);
-    product256(P, smem, buf0, 5, 4, P.x[1] + row0 * kH, kH, z2);
-    epilogue_silu(z2, P.bias[2], buf1);
-    // output layer, N = 64: warp w's 16 x 16 tile; then the loss gradient
+    for (int i = tid; i < 3 * kH + 64; i += kThreads) bias[i] = P.bias[i >> 8][i & 255];
+    Tile d0, d1, d2;   // products, then SiLU derivatives, of the hidden layers
+    product256(P, smem, buf0, 0, 1, nullptr, 0, d0);
+    epilogue_silu(d0, bias, buf1);
+    product256(P, smem, buf1, 1, 4, P.x[0] + row0 * kH, kH, d1);
+    epilogue_silu(d1, bias + kH, buf0);
+    product256(P, smem, buf0, 5, 4, P.x[1] + row0 * kH, kH, d2);
+    epilogue_silu(d2, bias + 2 * kH, buf1);
+    // output layer, N = 64: warp w's 16 x 8 tile; then the loss gradient
     {
-        float acc[2][4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) acc[i][k] = 0.f;
-        const int wm = (warp >> 2) * 16, wn = (warp & 3) * 16;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const int wm = (warp >> 3) * 16, wn = (warp & 7) * 8;
 #pragma unroll 1
         for (int q = 0; q < 4; ++q) {
             const int i = 9 + q;
@@ -226,45 +228,44 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
             if (q == 0) store_rows(buf1, P.x[2] + row0 * kH, kH);
             const unsigned char* st = smem + (i % kStages) * kStageBytes;
 #pragma unroll
-            for (int kk = 0; kk < 64; kk += 16) {
+            for (int kk = 0; kk < 64; kk += 32) {
                 uint32_t a[4], t[4];
+                const int r = kk + lane;   // four 8 x 8 matrices along k
+                ldsm_x4_t(t, st + r * 128 + (((wn >> 3) ^ (r & 7)) << 4));
                 ldsm_x4(a, buf1 + (wm + (lane & 15)) * kLdA + q * 64 + kk + (lane >> 4) * 8);
-                const int j = lane >> 3, r = kk + (lane & 7) + 8 * (j & 1), c = (wn >> 3) + (j >> 1);
-                ldsm_x4_t(t, st + r * 128 + ((c ^ (r & 7)) << 4));
-                mma_bf16(acc[0], a, t[0], t[1]);
-                mma_bf16(acc[1], a, t[2], t[3]);
+                mma_bf16(acc, a, t[0], t[1]);
+                ldsm_x4(a, buf1 + (wm + (lane & 15)) * kLdA + q * 64 + kk + 16 + (lane >> 4) * 8);
+                mma_bf16(acc, a, t[2], t[3]);
             }
         }
         const float scale = 1.f / (float)((size_t)P.batch * P.n_out);
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni)
+        for (int h = 0; h < 2; ++h) {
+            const int r = wm + (lane >> 2) + 8 * h, c = wn + (lane & 3) * 2;
+            float g[2];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int r = wm + (lane >> 2) + 8 * h, c = wn + ni * 8 + (lane & 3) * 2;
-                float g[2];
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    g[e] = 0.f;
-                    if (c + e < P.n_out) {
-                        const float z = acc[ni][2 * h + e] + P.bias[3][c + e];
-                        float tv = P.target[(row0 + r) * P.n_out + c + e];
-                        if (P.tmean) tv = (tv - P.tmean[c + e]) * P.tistd[c + e];
-                        const float d = z - tv;
-                        P.z3[(row0 + r) * 64 + c + e] = z;   // for the loss
-                        g[e] = 2.f * d * scale;
-                    }
+            for (int e = 0; e < 2; ++e) {
+                g[e] = 0.f;
+                if (c + e < P.n_out) {
+                    const float z = acc[2 * h + e] + bias[3 * kH + c + e];
+                    float tv = P.target[(row0 + r) * P.n_out + c + e];
+                    if (P.tmean) tv = (tv - P.tmean[c + e]) * P.tistd[c + e];
+                    const float d = z - tv;
+                    P.z3[(row0 + r) * 64 + c + e] = z;   // for the loss
+                    g[e] = 2.f * d * scale;
                 }
-                *reinterpret_cast<__nv_bfloat162*>(buf0 + r * kLdA + c) =
-                    __nv_bfloat162(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
             }
+            *reinterpret_cast<__nv_bfloat162*>(buf0 + r * kLdA + c) =
+                __nv_bfloat162(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
+        }
     }
-    float acc[2][4][4];
+    Tile acc;
     product256(P, smem, buf0, 13, 1, P.dz[3] + row0 * 64, 64, acc);
-    epilogue_grad(acc, z2, buf1);
+    epilogue_grad(acc, d2, buf1);
     product256(P, smem, buf1, 14, 4, P.dz[2] + row0 * kH, kH, acc);
-    epilogue_grad(acc, z1, buf0);
+    epilogue_grad(acc, d1, buf0);
     product256(P, smem, buf0, 18, 4, P.dz[1] + row0 * kH, kH, acc);
-    epilogue_grad(acc, z0, buf1);
+    epilogue_grad(acc, d0, buf1);
     __syncthreads();
     store_rows(buf1, P.dz[0] + row0 * kH, kH);
 }
@@ -359,13 +360,16 @@ __device__ __forceinline__ void column_slab(float (&part)[32][33], const GradLay
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = slab * L.slab_rows, r1 = min(batch, r0 + L.slab_rows);
     const int c = c0 + lane;
+    float s[8];   // row groups warp, warp + 4, ...
 #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-        const int ty = warp * 8 + g;
-        float s = 0.f;
-        for (int r = r0 + ty; r < r1; r += 32) s += __bfloat162float(L.dz[(size_t)r * L.n + c]);
-        part[ty][lane] = s;
-    }
+    for (int g = 0; g < 8; ++g) s[g] = 0.f;
+#pragma unroll 2
+    for (int r = r0 + warp; r < r1; r += 32)
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+            if (r + 4 * g < r1) s[g] += __bfloat162float(L.dz[(size_t)(r + 4 * g) * L.n + c]);
+#pragma unroll
+    for (int g = 0; g < 8; ++g) part[warp + 4 * g][lane] = s[g];
     __syncthreads();
     if (warp == 0) {
         float t = 0.f;
@@ -414,7 +418,25 @@ __global__ void __launch_bounds__(train::kGradThreads) train_grads_kernel(const 
         float part[32][33];
         float red[kGradThreads];
     } S;
+    dependency_wait();
+    launch_dependents();
+    // the short CTAs first, so that they run beside the products
     int b = (int)blockIdx.x;
+    if (b < 256) {
+        loss_block(S.red, P, b);
+        return;
+    }
+    b -= 256;
+#pragma unroll 1
+    for (int l = 0; l < 4; ++l) {
+        const GradLayer& L = P.layer[l];
+        const int groups = L.n / 32, count = groups * L.slabs;
+        if (b < count) {
+            column_slab(S.part, L, (b % groups) * 32, b / groups, P.batch);
+            return;
+        }
+        b -= count;
+    }
 #pragma unroll 1
     for (int l = 0; l < 4; ++l) {
         const GradLayer& L = P.layer[l];
@@ -426,31 +448,41 @@ __global__ void __launch_bounds__(train::kGradThreads) train_grads_kernel(const 
         }
         b -= count;
     }
-#pragma unroll 1
-    for (int l = 0; l < 4; ++l) {
-        const GradLayer& L = P.layer[l];
-        const int groups = L.n / 32, count = groups * L.slabs;
-        if (b < count) {
-            column_slab(S.part, L, (b % groups) * 32, b / groups, P.batch);
-            return;
-        }
-        b -= count;
-    }
-    loss_block(S.red, P, b);
 }
 
 // ---------------------------------------------------------------- update
 namespace train {
-__device__ __forceinline__ float adamw(const UpdateParams& P, float* w, float* m, float* v, size_t i, float g, float wd)
+struct Moments {
+    float w, m, v;
+};
+
+__device__ __forceinline__ float adamw(const UpdateParams& P, const Moments& o, float* w, float* m, float* v, size_t i,
+                                       float g, float wd)
 {
-    const float mi = P.b1 * m[i] + (1.f - P.b1) * g;
-    const float vi = P.b2 * v[i] + (1.f - P.b2) * g * g;
+    const float mi = P.b1 * o.m + (1.f - P.b1) * g;
+    const float vi = P.b2 * o.v + (1.f - P.b2) * g * g;
     m[i] = mi;
     v[i] = vi;
     const float mh = mi / P.bc1, vh = vi / P.bc2;
-    const float wi = w[i] * (1.f - P.lr * wd) - P.lr * mh / (sqrtf(vh) + P.eps);
+    const float wi = o.w * (1.f - P.lr * wd) - P.lr * mh / (sqrtf(vh) + P.eps);
     w[i] = wi;
     return wi;
+}
+
+// p[0] + p[stride] + ... (n terms, summed in order), the terms' loads sixteen
+// at a time in flight: one at a time the sum waits for L2 n times.
+__device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int n)
+{
+    float s = 0.f;
+    for (int z0 = 0; z0 < n; z0 += 16) {
+        float t[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) t[j] = z0 + j < n ? p[(size_t)(z0 + j) * stride] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (z0 + j < n) s = z0 + j == 0 ? t[0] : s + t[j];
+    }
+    return s;
 }
 }  // namespace train
 
@@ -458,7 +490,10 @@ __device__ __forceinline__ float adamw(const UpdateParams& P, float* w, float* m
 // memory in 64-byte rows) or, the last four CTAs, one layer's biases.
 __global__ void __launch_bounds__(256) train_update_kernel(const UpdateParams P)
 {
+    using namespace train;
     __shared__ bf16 tile[8][34];
+    dependency_wait();
+    launch_dependents();
     int b = (int)blockIdx.x;
     const int tid = threadIdx.x;
 #pragma unroll 1
@@ -468,11 +503,10 @@ __global__ void __launch_bounds__(256) train_update_kernel(const UpdateParams P)
         if (b < count) {
             const int r = (b / tn) * 32 + (tid >> 3), c = (b % tn) * 8 + (tid & 7);
             const size_t i = (size_t)r * L.n + c, mn = (size_t)L.k * L.n;
-            float g = L.part[i];
-#pragma unroll 8
-            for (int z = 1; z < L.splits; ++z) g += L.part[z * mn + i];
+            const Moments o{L.w[i], L.mw[i], L.vw[i]};
+            const float g = ordered_sum(L.part + i, mn, L.splits);
             L.gw[i] = g;
-            const bf16 h = __float2bfloat16(train::adamw(P, L.w, L.mw, L.vw, i, g, P.wd));
+            const bf16 h = __float2bfloat16(adamw(P, o, L.w, L.mw, L.vw, i, g, P.wd));
             L.w16[i] = h;
             tile[tid & 7][tid >> 3] = h;
             __syncthreads();
@@ -483,10 +517,10 @@ __global__ void __launch_bounds__(256) train_update_kernel(const UpdateParams P)
     }
     const UpdateLayer& L = P.layer[b];
     for (int c = tid; c < L.n; c += 256) {
-        float g = 0.f;
-        for (int k = 0; k < L.slabs; ++k) g += L.col[(size_t)k * L.n + c];
+        const Moments o{L.b[c], L.mb[c], L.vb[c]};
+        const float g = 0.f + ordered_sum(L.col + c, L.n, L.slabs);   // from +0, as the general kernel
         L.gb[c] = g;
-        train::adamw(P, L.b, L.mb, L.vb, c, g, 0.0f);
+        adamw(P, o, L.b, L.mb, L.vb, c, g, 0.0f);
     }
 }
 
@@ -495,15 +529,28 @@ cudaError_t launch_train_step(const RowsParams& R, const GradsParams& G, const U
     cudaError_t e = cudaFuncSetAttribute(train_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)train::kRowsSmem);
     if (e != cudaSuccess) return e;
-    train_rows_kernel<<<R.batch / train::kRows, train::kThreads, train::kRowsSmem, s>>>(R);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int grads = 256, updates = 4;   // loss blocks; bias blocks
     for (const GradLayer& L : G.layer) grads += (L.k / 64) * (L.n / 64) * L.splits + (L.n / 32) * L.slabs;
     for (const UpdateLayer& L : U.layer) updates += (L.k / 32) * (L.n / 8);
-    train_grads_kernel<<<grads, train::kGradThreads, 0, s>>>(G);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    train_update_kernel<<<updates, 256, 0, s>>>(U);
-    return cudaGetLastError();
+    cudaLaunchAttribute chain{};
+    chain.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    chain.val.programmaticStreamSerializationAllowed = 1;
+    auto config = [&](int grid, int block, size_t smem) {
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3(grid);
+        c.blockDim = dim3(block);
+        c.dynamicSmemBytes = smem;
+        c.stream = s;
+        c.attrs = &chain;
+        c.numAttrs = 1;
+        return c;
+    };
+    cudaLaunchConfig_t c = config(R.batch / train::kRows, train::kThreads, train::kRowsSmem);
+    if ((e = cudaLaunchKernelEx(&c, train_rows_kernel, R)) != cudaSuccess) return e;
+    c = config(grads, train::kGradThreads, 0);
+    if ((e = cudaLaunchKernelEx(&c, train_grads_kernel, G)) != cudaSuccess) return e;
+    c = config(updates, 256, 0);
+    return cudaLaunchKernelEx(&c, train_update_kernel, U);
 }
 
 }  // namespace sfh
