@@ -644,8 +644,7 @@ typedef struct hydro_cable_node_forces {
  * relative to the current, split between its nodes; the end nodes' forces
  * doubled.  Cables whose mode is neither FLOATING nor SUBMERGED, and cables
  * whose node range does not lie within n_nodes_total, are left untouched.
- * x and v are [n_nodes_total][3] FP64.  Device pointers on `stream`; the
- * call keeps n_nodes_total x 72 bytes of scratch per context. */
+ * x and v are [n_nodes_total][3] FP64.  Device pointers on `stream`. */
 hydro_status hydro_cable_forces_device(hydro_ctx* ctx, const hydro_cable* d_cables, uint32_t n_cables,
                                        const double* d_x, const double* d_v, uint32_t n_nodes_total,
                                        const hydro_ocean* ocean, const hydro_settings* settings,

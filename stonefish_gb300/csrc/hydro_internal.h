@@ -181,8 +181,7 @@ cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, co
 cudaError_t launch_compound_step(const KParams& P, const CompoundParams& C, LaunchShape shape, int cut64,
                                  cudaStream_t s, uint32_t* launches);
 cudaError_t launch_cable(const hydro_cable* cables, uint32_t n_cables, uint32_t n_nodes_total, const double* x,
-                         const double* v, OceanDev o, SettingsDev st, double* seg, hydro_cable_node_forces* out,
-                         unsigned* bad, cudaStream_t s);
+                         const double* v, OceanDev o, SettingsDev st, hydro_cable_node_forces* out, cudaStream_t s);
 cudaError_t launch_fft_ocean(const float4* s12, const float4* s34, const int2* idx, const float2* w, int passes,
                              float4 inv_grid, float t, float4* out, cudaStream_t s);
 cudaError_t launch_mesh_props(const TileDesc* tiles, uint32_t first_tile, uint32_t n_tiles, int pass, double thickness,

@@ -262,6 +262,44 @@ def test_jet_and_pipe_currents(oracle, hctx, sphere_run):
         assert np.max(v[cross]) < 1e-5, k
 
 
+@pytest.mark.parametrize("where,axis", [((0.0, 0.0), (1.0, 0.0, 0.0)), ((700.0, -450.0), (0.6, 0.8, 0.0)),
+                                        ((30.0, 20.0), (0.0, 3.0, 0.0))])
+def test_field_current_edges(oracle, hctx, sphere_run, where, axis):
+    """Spheres across the edges of a jet (side and nozzle) and a pipe (side and
+    both ends), near and far from the world origin and with an axis that is not
+    of unit length: faces that the FP32 bound sends past the currents and those
+    that evaluate them, against the oracle, which evaluates every one.  Same
+    1e-5 as test_jet_and_pipe_currents (exp and pow of two libraries)."""
+    sc = sphere_run
+    d = np.asarray(axis)
+    oc = scenarios.flat_ocean((0.1, 0.0, 0.0))
+    oc.n_currents = 3
+    for i, (typ, point) in enumerate(((abi.CURRENT_JET, (where[0] - 2.0, where[1], 0.2)),
+                                      (abi.CURRENT_PIPE, (where[0], where[1] - 2.0, 0.1)))):
+        c = oc.currents[1 + i]
+        c.type, c.enabled, c.radius, c.radius2, c.length, c.speed, c.gamma = typ, 1, 0.4, 0.9, 4.0, 1.5, 0.7
+        c.point[:] = point
+        c.dir[:] = axis
+    bodies = sc["bodies"][:64].copy()
+    rng = np.random.default_rng(3)
+    n = len(bodies)
+    u = d / np.linalg.norm(d)
+    side = np.array([-u[1], u[0], 0.0])
+    xy = np.asarray([*where, 0.0]) + rng.uniform(-3.5, 5.5, (n, 1)) * u + rng.uniform(-2.0, 2.0, (n, 1)) * side
+    for k in (0, 1):
+        shift = xy[:, k] - bodies["T_CG"]["origin"][:, k]
+        for f in ("aabb_min", "aabb_max"):
+            bodies[f][:, k] += shift
+        bodies["T_CG"]["origin"][:, k] = bodies["T_C"]["origin"][:, k] = xy[:, k]
+    sub = {"meshes": sc["meshes"], "bodies": bodies, "ocean": oc, "_ids": sc["_ids"]}
+    gpu = run_batch(hctx, sub)
+    mir = run_oracle(oracle, MIRROR32, sub)
+    cross = gpu["position"] == abi.CROSSING_SURFACE
+    assert cross.sum() > 20
+    for k, v in scaled_errors(gpu, mir, body_lengths(sub)).items():
+        assert np.max(v[cross]) < 1e-5, k
+
+
 # ------------------------------------------------------------- batches
 @pytest.mark.parametrize("cut", ["fp64", "fp32"])
 def test_mixed_batch_matches_mirror(oracle, hctx, hctx64, cut):
