@@ -3,35 +3,42 @@
 // layers (16 -> 256 -> 256 -> 256 -> 16) with the activations kept in shared
 // memory and the accumulators in tensor memory.
 //
-//   * persistent: one CTA per SM loops over the blocks; the next block's
-//     features are loaded into registers while the current block runs, and
-//     its first-layer weights are copied while the last layer runs;
-//   * operands are K-major BF16 in the 128-byte-swizzled canonical layout
+//   * persistent: a CTA per SM loops over pairs of 128-state blocks, both in
+//     flight: while one block's epilogue runs, the tensor pipe works for the
+//     other.  One block alone leaves the MUFU (one tanh per activation) idle
+//     while its MMAs, their commits and waits run, a quarter of the time;
+//   * each block has 128 accumulator columns and 128 columns of tensor
+//     memory with its activations, two BF16 to a column, as the A operand:
+//     an MMA then reads only its weights from shared memory (with the
+//     activations there too, an M = 128, N = 256, K = 16 instruction caused 24
+//     KB of shared-memory traffic, 190 cycles' worth for 128 of arithmetic);
+//   * a layer runs as two halves of N = 128 columns.  The first half's
+//     results wait in registers, since the activations they replace are still
+//     the second half's operand, and both halves are written after it;
+//   * weights are K-major BF16 in the 128-byte-swizzled canonical layout
 //     (8-row x 128-byte atoms, 16-byte chunk c of row r stored at chunk
-//     c ^ (r % 8)); each [rows x 64] K-block is contiguous, blocks follow
-//     each other;
-//   * the weights are packed once into that image in global memory
-//     (pack_sw128_kernel), so each layer's weights arrive with one 1-D bulk
-//     copy (cp.async.bulk, mbarrier complete_tx) while the previous layer's
-//     epilogue runs;
-//   * one lane of a dedicated warp issues tcgen05.mma (M = 128, N = 256 or
-//     16, K = 16 per instruction, FP32 accumulate) and commits to an
-//     mbarrier; the accumulators of consecutive layers alternate between
-//     the two halves of 512 TMEM columns;
-//   * sixteen epilogue warps read a layer's accumulator with tcgen05.ld
-//     (warp w reads TMEM lanes 32 (w % 4) .. +31), one 64-column K-block
-//     at a time, add the bias, apply SiLU, round to BF16 and write that
-//     K-block of the next layer's A operand, then arrive on the K-block's
-//     mbarrier: the next layer's MMAs on K-block g start while the
-//     epilogue works on K-blocks g + 1 ..;
-//   * the next layer's weights stream in as four K-block copies, each on
-//     its own mbarrier, as soon as the current layer's MMAs have retired;
-//   * the input features are normalised and rounded in the kernel, the
-//     output (bias added) is written as FP32 rows of 16.
+//     c ^ (r % 8)), packed once into that image in global memory
+//     (pack_sw128_kernel).  The second layer's 128 KB and the last layer's
+//     stay in shared memory; the first and third layers' stream through five
+//     16 KB slots (64 columns of K by half the rows, contiguous in the
+//     image) by 1-D bulk copies that a warp of its own keeps ahead, each
+//     used for both blocks;
+//   * one lane of a warp issues tcgen05.mma (FP32 accumulate);
+//   * eight epilogue warps per block read its accumulator with tcgen05.ld
+//     (warp w reads TMEM lanes 32 (w % 4) .. +31), add the bias, apply SiLU,
+//     round to BF16 and write the next A operand with tcgen05.st;
+//   * four more warps write the output rows (FP32 rows of 16, bias added) and
+//     the next pair's features, loaded, normalised and rounded ahead.
+//
+// Bound: MUFU (2,048 cycles per block and hidden layer) and the tensor pipe
+// (2,112), each with its hand-over: half a layer takes 1,450 cycles of either.
+// 65,536 states: 36.8 us with one block in flight and its activations in
+// shared memory, 26.7 us now (671 TFLOP/s, 34% of the measured 1,954).
 //
 // Every mbarrier wait is bounded (%globaltimer); a timeout sets *err, the
-// CTA stops issuing work, waits (bounded) for its tensor-core work to
-// retire, frees its tensor memory and returns.
+// CTA stops issuing work, waits (bounded) for its tensor-core work and its
+// copies to retire, frees its tensor memory and returns.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -49,17 +56,39 @@ constexpr int kHid = 256;
 constexpr int kIn = 16;         // features = layer-0 K
 constexpr int kOut = 16;        // output columns (6 used)
 constexpr int kEpiWarps = 16;                   // epilogue warps
-constexpr int kThreads = (kEpiWarps + 1) * 32;  // + one MMA warp
-constexpr uint32_t kTmemCols = 512;             // two 256-column accumulators
+constexpr int kThreads = (kEpiWarps + 6) * 32;  // + MMA warp + weight-copy warp + four in/out warps
+constexpr uint32_t kTmemCols = 512;
 
 // shared-memory image (offsets from a 1024-byte-aligned base)
-constexpr uint32_t kOffA = 0;                        // 128 x 256 bf16, 4 K-blocks of 16 KB
-constexpr uint32_t kOffW = kOffA + 4 * 16384;        // 256 x 256 bf16, 4 K-blocks of 32 KB
-constexpr uint32_t kOffW3 = kOffW + 4 * 32768;       // 16 x 256 bf16, 4 K-blocks of 2 KB
+constexpr uint32_t kSlots = 5;
+constexpr uint32_t kOffW1 = 0;                       // second layer: 256 x 256 bf16, 4 K-blocks of 32 KB
+constexpr uint32_t kOffRing = kOffW1 + 4 * 32768;    // 128 weight rows x 64 columns of K per slot
+constexpr uint32_t kOffW3 = kOffRing + kSlots * 16384;   // 16 x 256 bf16, 4 K-blocks of 2 KB
 constexpr uint32_t kOffBias = kOffW3 + 4 * 2048;     // 3 x 256 + 16 floats
-constexpr uint32_t kOffBar = kOffBias + (3 * kHid + kOut) * 4;   // 11 mbarriers
-constexpr uint32_t kOffTmem = kOffBar + 12 * 8;
+constexpr int kNormOff = 3 * kHid + kOut;            // feature means and inverse deviations
+constexpr uint32_t kOffBar = kOffBias + (kNormOff + 2 * kIn) * 4;
+constexpr uint32_t kBarRoom = 32 * 8;
+constexpr uint32_t kOffTmem = kOffBar + kBarRoom;
 constexpr uint32_t kSmemBytes = kOffTmem + 16 + 1024; // + alignment slack
+static_assert(kSmemBytes <= 227 * 1024, "one CTA per SM");
+
+// tensor memory columns of block t: accumulator, A operand
+constexpr uint32_t kColD = 0, kColA = 256;      // + 128 t
+
+// mbarriers (byte offsets from kOffBar; [2]: one per block in flight)
+enum : uint32_t {
+    kBarFull = 0,                         // [kSlots] a weight slot has arrived
+    kBarFree = kBarFull + 8 * kSlots,     // [kSlots] the MMAs that read a slot have retired
+    kBarD = kBarFree + 8 * kSlots,        // [2] half a hidden layer is in the accumulator
+    kBarOut = kBarD + 16,                 // [2] the output layer is
+    kBarDrained = kBarOut + 16,           // [2] the first half has been read from the accumulator
+    kBarAct = kBarDrained + 16,           // [2] the second half too, and the next A operand is written
+    kBarIn = kBarAct + 16,                // [2] the output has been read, the next features are written
+    kBarW1 = kBarIn + 16,                 // [4] a K-block of the second layer's weights
+    kBarFixed = kBarW1 + 32,              // the last layer's weights; at the end the last MMAs
+    kBarEnd = kBarFixed + 8
+};
+static_assert(kBarEnd <= kBarRoom, "mbarrier room");
 
 // global weight image (bytes)
 constexpr uint32_t kImgW0 = 0;                       // 256 x 64 (K 16 used) = 32 KB
@@ -113,16 +142,18 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
-// bounded wait: gives up after limit_ns
+// Bounded wait: gives up after limit_ns.  A try suspends the thread in
+// hardware until the phase completes or a system-dependent time passes;
+// sleeping between tries instead woke up to 1,700 cycles late.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns)
 {
     if (mbar_try(bar, parity)) return true;
     const uint64_t t0 = globaltimer();
-    while (!mbar_try(bar, parity)) {
+    for (;;) {
+        for (int i = 0; i < 16; ++i)
+            if (mbar_try(bar, parity)) return true;
         if (globaltimer() - t0 > limit_ns) return false;
-        __nanosleep(64);
     }
-    return true;
 }
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
@@ -136,11 +167,23 @@ __device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
 }
 
-__device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+// D[tmem_d] (+)= A[tmem_a] B[desc b]
+__device__ __forceinline__ void mma(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t idesc, uint32_t acc)
 {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                 :: "r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                 :: "r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+}
+
+// One lane of a converged warp, in a form that the compiler knows to be a
+// single one: behind a plain lane test every tcgen05.mma moved its operands
+// to uniform registers by a loop over the active lanes and took 160 to 200
+// cycles to issue, more than its 66 (N = 128) to execute.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t bar)
@@ -151,7 +194,6 @@ __device__ __forceinline__ void mma_commit(uint32_t bar)
 
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
 {
@@ -167,43 +209,36 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
 {
-    uint32_t r[32];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                  "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
                    "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
                    "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
                    "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
                    "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+                 : "r"(taddr) : "memory");
 }
 
-// Split form of tmem_ld16 for software pipelining: the load is issued
-// without waiting, and the wait names the destination registers as in-out
-// operands so that no use of them can be scheduled before it.
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16])
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16])
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                   "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr));
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+                 "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
+                 "tcgen05.wait::st.sync.aligned;"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+                    "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
+                    "r"(r[15]) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16])
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
 {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
-                   "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]),
-                   "+r"(r[14]), "+r"(r[15])
-                 :: "memory");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
+                 "tcgen05.wait::st.sync.aligned;"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b)
@@ -217,109 +252,64 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
 }
 
-// A hidden layer's epilogue, one K-block (64 columns) at a time: D (TMEM)
-// + bias -> SiLU -> BF16 -> columns 64 g .. of the A operand (row = TMEM
-// lane), then an arrival on K-block g's mbarrier so that the next layer's
-// MMAs on it can start.  Warp w: lanes 32 (w % 4).., columns
-// 64 g + 16 (w / 4) ..; the tensor-memory load of K-block g + 1 is in
-// flight while K-block g is converted.
-__device__ __forceinline__ void hidden_epilogue(uint32_t acc, unsigned char* base, const float* bias, uint32_t abar)
+// 32 accumulator columns col .. of this warp's rows: bias, then SiLU(z) =
+// z sigmoid(z) = u + u tanh(u) with u = z / 2, two columns at a time with
+// the packed FP32 instructions (each half rounds as the scalar operation
+// would); one hardware tanh (tanh.approx.f32, relative error about 2^-11) per
+// value, so the absolute error is at most |z| 2^-12, below the BF16 rounding
+// that follows.
+__device__ __forceinline__ void silu32(const uint32_t (&z)[32], const float* bias, uint32_t (&w)[16])
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t q = (uint32_t)(warp & 3), sub = (uint32_t)(warp >> 2);
-    const uint32_t row = 32u * q + (uint32_t)lane;
-    const uint32_t lanes = (32u * q) << 16;
-    uint32_t cur[16], nxt[16];
-    tmem_ld16_issue(acc + lanes + 16u * sub, cur);
-    tmem_ld_wait(cur);
 #pragma unroll
-    for (uint32_t g = 0; g < 4; ++g) {
-        const uint32_t col = 64u * g + 16u * sub;
-        if (g < 3) tmem_ld16_issue(acc + lanes + col + 64u, nxt);
-        uint32_t w[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            // bias, then SiLU(z) = z sigmoid(z) = h + h tanh(h) with h = z / 2,
-            // on two columns at a time with the packed FP32 instructions (each
-            // half rounds as the scalar operation would): one hardware tanh
-            // (tanh.approx.f32, relative error about 2^-11) per value, so the
-            // absolute error is at most |z| 2^-12, below the BF16 rounding of
-            // the activation that follows
-            const float2 b2 = *reinterpret_cast<const float2*>(bias + col + 2 * i);
-            const float2 z2 = __fadd2_rn(make_float2(__uint_as_float(cur[2 * i]), __uint_as_float(cur[2 * i + 1])), b2);
-            const float2 h2 = __fmul2_rn(z2, make_float2(0.5f, 0.5f));
-            float t0, t1;
-            asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(h2.x));
-            asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(h2.y));
-            const float2 s2 = __ffma2_rn(h2, make_float2(t0, t1), h2);
-            w[i] = pack2(s2.x, s2.y);
-        }
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-            *reinterpret_cast<uint4*>(base + kOffA + sw128_offset(kRows, row, col + 8u * c)) =
-                make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
-        fence_async_smem();
-        mbar_arrive(abar + 8u * g);
-        if (g < 3) {
-            tmem_ld_wait(nxt);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) cur[i] = nxt[i];
-        }
+    for (int i = 0; i < 16; ++i) {
+        const float2 b2 = *reinterpret_cast<const float2*>(bias + 2 * i);
+        const float2 z2 = __fadd2_rn(make_float2(__uint_as_float(z[2 * i]), __uint_as_float(z[2 * i + 1])), b2);
+        const float2 u2 = __fmul2_rn(z2, make_float2(0.5f, 0.5f));
+        float t0, t1;
+        asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(u2.x));
+        asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(u2.y));
+        const float2 s2 = __ffma2_rn(u2, make_float2(t0, t1), u2);
+        w[i] = pack2(s2.x, s2.y);
     }
-    fence_before();
 }
 
 }  // namespace tc
 
-// Normalised BF16 inputs of one 128-state block: thread t < 256 holds row
-// t % 128, features 8 (t / 128) .. + 7.
-__device__ __forceinline__ void load_features(const float* __restrict__ feats, uint32_t n, uint32_t row0,
-                                              const float* __restrict__ fmean, const float* __restrict__ fistd,
-                                              float (&x)[8])
-{
-    using namespace tc;
-    const uint32_t r = threadIdx.x & (kRows - 1), h = threadIdx.x >> 7;
-    const uint32_t gr = row0 + r;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int k = (int)h * 8 + j;
-        x[j] = gr < n ? (feats[(size_t)gr * kIn + k] - fmean[k]) * fistd[k] : 0.f;
-    }
-}
+// One network's parameters and output.
+struct MlpNet {
+    const float* fmean;
+    const float* fistd;
+    const unsigned char* wimg;
+    const float* b[4];
+    float* out;
+};
 
-__device__ __forceinline__ void store_features(unsigned char* base, const float (&x)[8])
-{
-    using namespace tc;
-    const uint32_t r = threadIdx.x & (kRows - 1), h = threadIdx.x >> 7;
-    *reinterpret_cast<uint4*>(base + kOffA + sw128_offset(kRows, r, h * 8)) =
-        make_uint4(pack2(x[0], x[1]), pack2(x[2], x[3]), pack2(x[4], x[5]), pack2(x[6], x[7]));
-}
+struct MlpParams {
+    const float* feats;
+    uint32_t n;
+    uint32_t n_nets;
+    uint32_t in_flight;   // blocks per CTA at a time, 1 or 2
+    MlpNet net[2];
+    unsigned* err;
+};
 
-// Persistent: CTA c takes the 128-state blocks c, c + gridDim.x, ...; the
-// tensor memory, the mbarriers, the biases and the last layer's weights are
-// set up once.  While a block runs, the epilogue threads hold the next
-// block's features in registers and write them once the block's last MMAs
-// have retired; the next block's first-layer weights are copied as soon as
-// the weight buffer is free.
-__global__ void __launch_bounds__(tc::kThreads, 1)
-mlp_tc_kernel(const float* __restrict__ feats, uint32_t n, const float* __restrict__ fmean,
-              const float* __restrict__ fistd, const unsigned char* __restrict__ wimg,
-              const float* __restrict__ b0, const float* __restrict__ b1, const float* __restrict__ b2,
-              const float* __restrict__ b3, float* __restrict__ out, unsigned* __restrict__ err)
+// CTA c works for network c % n_nets on the groups of in_flight 128-state
+// blocks c / n_nets, + gridDim.x / n_nets, ...  (the grid is a multiple of
+// n_nets).
+__global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_constant__ MlpParams P)
 {
     using namespace tc;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-    const uint32_t sb = smem_u32(base);
-    // mbarriers: first-layer weights; MMA commits; the four K-block copies of
-    // a hidden layer's weights; the four K-blocks of A; a block's features
-    const uint32_t barW0 = sb + kOffBar, barM = barW0 + 8, wbar = barW0 + 16, abar = barW0 + 48,
-                   barF = barW0 + 80;
+    const uint32_t sb = smem_u32(base), bars = sb + kOffBar;
     float* bias = reinterpret_cast<float*>(base + kOffBias);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + kOffTmem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t n_blocks = (n + kRows - 1) / kRows;
+    const MlpNet& N = P.net[blockIdx.x % P.n_nets];
+    const uint32_t n_blocks = (P.n + kRows - 1) / kRows, both = P.in_flight;
+    const uint32_t n_groups = (n_blocks + both - 1) / both;
+    const uint32_t first = blockIdx.x / P.n_nets, stride = gridDim.x / P.n_nets;
     const uint64_t kLimit = 1000000000ull;   // 1 s per wait
 
     if (warp == 0) {
@@ -328,160 +318,74 @@ mlp_tc_kernel(const float* __restrict__ feats, uint32_t n, const float* __restri
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(barW0) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(barM) : "memory");
-        for (uint32_t g = 0; g < 4; ++g) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(wbar + 8u * g) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(abar + 8u * g), "r"(kEpiWarps * 32)
-                         : "memory");
+        for (uint32_t b = 0; b < kBarEnd; b += 8) {
+            const uint32_t count = b >= kBarDrained && b < kBarIn ? 8u : b >= kBarIn && b < kBarW1 ? 4u : 1u;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bars + b), "r"(count) : "memory");
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(barF), "r"(kEpiWarps * 32) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = tid; i < kHid; i += kThreads) {
+        bias[i] = N.b[0][i];
+        bias[kHid + i] = N.b[1][i];
+        bias[2 * kHid + i] = N.b[2][i];
+    }
+    if (tid < kOut) bias[3 * kHid + tid] = N.b[3][tid];
+    if (tid < kIn) {
+        bias[kNormOff + tid] = N.fmean[tid];
+        bias[kNormOff + kIn + tid] = N.fistd[tid];
     }
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // the first block's first-layer weights and the last layer's (which stay)
-    if (tid == 0) {
-        expect_tx(barW0, 32768u + 8192u);
-        bulk_load(sb + kOffW, wimg + kImgW0, 32768u, barW0);
-        bulk_load(sb + kOffW3, wimg + kImgW3, 8192u, barW0);
-    }
-    for (int i = tid; i < kHid; i += kThreads) {
-        bias[i] = b0[i];
-        bias[kHid + i] = b1[i];
-        bias[2 * kHid + i] = b2[i];
-    }
-    if (tid < kOut) bias[3 * kHid + tid] = b3[tid];
-    float x[8];
-    if (tid < kRows * (kIn / 8)) {
-        load_features(feats, n, blockIdx.x * (uint32_t)kRows, fmean, fistd, x);
-        store_features(base, x);
-    }
-    fence_async_smem();
-    __syncthreads();
-
     bool ok = true;
-    if (warp == kEpiWarps) {
-        // ---- MMA warp: one lane issues every layer's MMAs and the weight copies
-        if (lane == 0) {
-            const uint32_t id_hid = idesc_bf16(128, 256), id_out = idesc_bf16(128, kOut);
-            uint32_t w_pending = 0, w_par = 0;    // K-block copies issued and not yet waited for; their parity
-            uint32_t w0_pending = 1, w0_par = 0;  // first-layer copy issued and not yet waited for; its parity
-            uint32_t commits = 0, seen = 0;   // barM phases committed / observed complete
-            uint32_t a_done = 0;              // completions of the A K-block barriers waited for
-            uint32_t k = 0;
-#pragma unroll 1
-            for (uint32_t blk = blockIdx.x; blk < n_blocks && ok; blk += gridDim.x, ++k) {
-                ok = mbar_wait(barW0, k & 1u, kLimit);
-                if (ok) w0_pending = 0;
-                // this block's features: written once the epilogue has seen
-                // the previous block's last commit
-                if (ok && k > 0) {
-                    ok = mbar_wait(barF, (k - 1u) & 1u, kLimit);
-                    if (ok) ++seen;
-                }
-                if (!ok) break;
-                fence_after();
-                mma(tmem, sw128_desc(sb + kOffA), sw128_desc(sb + kOffW), id_hid, 0u);   // layer 0: K = 16
-                mma_commit(barM);
-                ++commits;
-#pragma unroll 1
-                for (uint32_t l = 1; l <= 3 && ok; ++l) {
-                    // layer l - 1's MMAs have retired: the weight buffer takes
-                    // layer l's weights (or, before the last layer, the next
-                    // block's first-layer weights)
-                    ok = mbar_wait(barM, (l - 1u) & 1u, kLimit);
-                    if (!ok) break;
-                    ++seen;
-                    if (l < 3) {
-                        for (uint32_t g = 0; g < 4; ++g) {
-                            expect_tx(wbar + 8u * g, 32768u);
-                            bulk_load(sb + kOffW + 32768u * g, wimg + (l == 1 ? kImgW1 : kImgW2) + 32768u * g,
-                                      32768u, wbar + 8u * g);
-                        }
-                        w_pending = 0xFu;
-                        w_par = (l - 1u) & 1u;
-                    } else if (blk + gridDim.x < n_blocks) {
-                        expect_tx(barW0, 32768u);
-                        bulk_load(sb + kOffW, wimg + kImgW0, 32768u, barW0);
-                        w0_pending = 1;
-                        w0_par = (k + 1u) & 1u;
-                    }
-                    const uint32_t acc = tmem + 256u * (l & 1u);
-#pragma unroll 1
-                    for (uint32_t g = 0; g < 4 && ok; ++g) {
-                        if (l < 3) {
-                            ok = mbar_wait(wbar + 8u * g, (l - 1u) & 1u, kLimit);
-                            if (!ok) break;
-                            w_pending &= ~(1u << g);
-                        }
-                        ok = mbar_wait(abar + 8u * g, a_done & 1u, kLimit);   // K-block g of layer l's input
-                        if (!ok) break;
-                        fence_after();
+    if (warp >= kEpiWarps + 2) {
+        // ---- in/out warps: warp with quadrant q holds rows 32 q .. +31
+        const uint32_t lanes = (32u * (uint32_t)(warp & 3)) << 16, row = 32u * (uint32_t)(warp & 3) + (uint32_t)lane;
+        uint32_t x[2][8];
+        auto load_in = [&](uint32_t t, uint32_t group) {
+            const uint32_t gr = (both * group + t) * (uint32_t)kRows + row;
+            const float* mean = bias + kNormOff;
+            const float* istd = mean + kIn;
+            float v[kIn];
 #pragma unroll
-                        for (uint32_t j = 0; j < 4; ++j) {
-                            const uint32_t off_a = kOffA + g * (kRows * 128u) + j * 32u;
-                            if (l < 3) {
-                                const uint32_t off_b = kOffW + g * (kHid * 128u) + j * 32u;
-                                mma(acc, sw128_desc(sb + off_a), sw128_desc(sb + off_b), id_hid, (g | j) ? 1u : 0u);
-                            } else {
-                                const uint32_t off_b = kOffW3 + g * (kOut * 128u) + j * 32u;
-                                mma(acc, sw128_desc(sb + off_a), sw128_desc(sb + off_b), id_out, (g | j) ? 1u : 0u);
-                            }
-                        }
-                    }
-                    if (!ok) break;
-                    ++a_done;
-                    mma_commit(barM);
-                    ++commits;
-                }
-                // the epilogue waits for the last layer's commit; this warp
-                // counts it as seen once the next block's features arrive
+            for (int k = 0; k < kIn; ++k) v[k] = gr < P.n ? (P.feats[(size_t)gr * kIn + k] - mean[k]) * istd[k] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[t][k] = pack2(v[2 * k], v[2 * k + 1]);
+        };
+        auto store_in = [&](uint32_t t) {
+            tmem_st8(tmem + kColA + 128u * t + lanes, x[t]);
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + kBarIn + 8u * t);
+        };
+#pragma unroll
+        for (uint32_t t = 0; t < 2; ++t)
+            if (t < both) {
+                load_in(t, first);
+                store_in(t);
             }
-            if (!ok) {
-                // let issued tensor-core work and copies retire before the
-                // tensor memory is freed and the CTA exits (bounded): one more
-                // commit, then the barrier's phases in order
-                atomicOr(err, 1u);
-                mma_commit(barM);
-                ++commits;
-                for (uint32_t c = seen; c < commits; ++c) mbar_wait(barM, c & 1u, kLimit);
-                for (uint32_t g = 0; g < 4; ++g)
-                    if ((w_pending >> g) & 1u) mbar_wait(wbar + 8u * g, w_par, kLimit);
-                if (w0_pending) mbar_wait(barW0, w0_par, kLimit);
-            }
-        }
-        __syncwarp();
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-    } else {
-        // ---- epilogue warps
+        uint32_t k = 0;
 #pragma unroll 1
-        for (uint32_t blk = blockIdx.x; blk < n_blocks && ok; blk += gridDim.x) {
-            const uint32_t next = blk + gridDim.x;
-            if (tid < kRows * (kIn / 8)) {
-                if (next < n_blocks) load_features(feats, n, next * (uint32_t)kRows, fmean, fistd, x);
-            }
-            // layers 0..2 feed the next layer K-block by K-block
-#pragma unroll 1
-            for (uint32_t l = 0; l < 3 && ok; ++l) {
-                ok = mbar_wait(barM, l & 1u, kLimit);
+        for (uint32_t group = first; group < n_groups && ok; group += stride, ++k) {
+            const bool more = group + stride < n_groups;
+#pragma unroll
+            for (uint32_t t = 0; t < 2; ++t)
+                if (more && t < both) load_in(t, group + stride);
+#pragma unroll
+            for (uint32_t t = 0; t < 2; ++t) {
+                const uint32_t blk = both * group + t;
+                if (t >= both || blk >= n_blocks || !ok) break;
+                ok = mbar_wait(bars + kBarOut + 8u * t, k & 1u, kLimit);
                 if (!ok) break;
                 fence_after();
-                hidden_epilogue(tmem + 256u * (l & 1u), base, bias + l * kHid, abar);
-            }
-            // output layer: N = 16, bias, FP32 rows of 16
-            if (ok) ok = mbar_wait(barM, 1u, kLimit);
-            if (!ok) break;
-            fence_after();
-            if (warp < 4) {
                 float v[16];
-                tmem_ld16(tmem + 256u + ((32u * (uint32_t)warp) << 16), v);
-                const uint32_t gr = blk * (uint32_t)kRows + 32u * (uint32_t)warp + (uint32_t)lane;
-                if (gr < n) {
-                    float4* o = reinterpret_cast<float4*>(out + (size_t)gr * kOut);
+                tmem_ld16(tmem + kColD + 128u * t + lanes, v);
+                if (more) store_in(t);
+                const uint32_t gr = blk * (uint32_t)kRows + row;
+                if (gr < P.n) {
+                    float4* o = reinterpret_cast<float4*>(N.out + (size_t)gr * kOut);
                     const float* bb = bias + 3 * kHid;
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
@@ -489,15 +393,171 @@ mlp_tc_kernel(const float* __restrict__ feats, uint32_t n, const float* __restri
                                            v[4 * i + 2] + bb[4 * i + 2], v[4 * i + 3] + bb[4 * i + 3]);
                 }
             }
-            // the next block's features into A (its last MMAs have retired)
-            if (next < n_blocks) {
-                if (tid < kRows * (kIn / 8)) store_features(base, x);
+        }
+        if (!ok && lane == 0) atomicOr(P.err, 1u);
+    } else if (warp == kEpiWarps + 1) {
+        // ---- weight copies, in the order the MMA warp uses them
+        if (elect_one()) {
+            uint32_t use = 0;
+            auto copy = [&](const unsigned char* src) {
+                const uint32_t s = use % kSlots;
+                if (ok && use >= kSlots) ok = mbar_wait(bars + kBarFree + 8u * s, (use / kSlots - 1u) & 1u, kLimit);
+                if (!ok) return;
+                expect_tx(bars + kBarFull + 8u * s, 16384u);
+                bulk_load(sb + kOffRing + 16384u * s, src, 16384u, bars + kBarFull + 8u * s);
+                ++use;
+            };
+#pragma unroll 1
+            for (uint32_t group = first; group < n_groups && ok; group += stride) {
+                copy(N.wimg + kImgW0);
+                copy(N.wimg + kImgW0 + 16384u);
+                if (group == first) {
+                    for (uint32_t g = 0; g < 4; ++g) {
+                        expect_tx(bars + kBarW1 + 8u * g, 32768u);
+                        bulk_load(sb + kOffW1 + 32768u * g, N.wimg + kImgW1 + 32768u * g, 32768u, bars + kBarW1 + 8u * g);
+                    }
+                    expect_tx(bars + kBarFixed, 8192u);
+                    bulk_load(sb + kOffW3, N.wimg + kImgW3, 8192u, bars + kBarFixed);
+                }
+#pragma unroll 1
+                for (uint32_t i = 0; i < 8; ++i)   // half i / 4, K-block i % 4
+                    copy(N.wimg + kImgW2 + 32768u * (i & 3u) + 16384u * (i >> 2));
+            }
+            // every copy has landed before the CTA may end (bounded)
+            for (uint32_t u = use > kSlots ? use - kSlots : 0u; u < use; ++u)
+                if (!mbar_wait(bars + kBarFull + 8u * (u % kSlots), (u / kSlots) & 1u, kLimit)) ok = false;
+            if (!ok) atomicOr(P.err, 1u);
+        }
+        __syncwarp();
+    } else if (warp == kEpiWarps) {
+        // ---- MMA warp: one lane issues every MMA
+        if (elect_one()) {
+            const uint32_t id_half = idesc_bf16(128, 128), id_out = idesc_bf16(128, kOut);
+            const uint64_t ring = sw128_desc(sb + kOffRing), w1 = sw128_desc(sb + kOffW1), w3 = sw128_desc(sb + kOffW3);
+            uint32_t use = 0, k = 0;
+            bool fixed = false;
+#pragma unroll 1
+            for (uint32_t group = first; group < n_groups && ok; group += stride, ++k) {
+                const uint32_t nt = min(both, n_blocks - both * group);
+                // first layer, K = 16
+#pragma unroll 1
+                for (uint32_t h = 0; h < 2 && ok; ++h, ++use) {
+                    const uint32_t s = use % kSlots;
+                    ok = mbar_wait(bars + kBarFull + 8u * s, (use / kSlots) & 1u, kLimit);
+#pragma unroll 1
+                    for (uint32_t t = 0; t < nt && ok; ++t) {
+                        ok = h == 0 ? mbar_wait(bars + kBarIn + 8u * t, k & 1u, kLimit)
+                                    : mbar_wait(bars + kBarDrained + 8u * t, (3u * k) & 1u, kLimit);
+                        if (!ok) break;
+                        fence_after();
+                        mma(tmem + kColD + 128u * t, tmem + kColA + 128u * t, ring + 1024u * s, id_half, 0u);
+                        mma_commit(bars + kBarD + 8u * t);
+                    }
+                    mma_commit(bars + kBarFree + 8u * s);
+                }
+#pragma unroll 1
+                for (uint32_t lh = 2; lh < 6 && ok; ++lh) {   // layer lh / 2, half lh % 2
+                    const uint32_t l = lh >> 1, h = lh & 1u;
+#pragma unroll 1
+                    for (uint32_t t = 0; t < nt && ok; ++t) {
+                        // block t's operand is written and its accumulator free
+                        ok = h == 0 ? mbar_wait(bars + kBarAct + 8u * t, (3u * k + l - 1u) & 1u, kLimit)
+                                    : mbar_wait(bars + kBarDrained + 8u * t, (3u * k + l) & 1u, kLimit);
+                        if (!ok) break;
+                        fence_after();
+                        const uint32_t d = tmem + kColD + 128u * t, a = tmem + kColA + 128u * t;
+#pragma unroll 1
+                        for (uint32_t g = 0; g < 4; ++g) {
+                            const uint32_t s = (use + g) % kSlots;
+                            uint64_t w = w1 + 2048u * g + 1024u * h;   // descriptors count 16 bytes
+                            if (l == 1 && !fixed) {   // the first group's second layer
+                                ok = mbar_wait(bars + kBarW1 + 8u * g, 0u, kLimit);
+                                if (!ok) break;
+                            }
+                            if (l == 2) {
+                                w = ring + 1024u * s;
+                                if (t == 0) ok = mbar_wait(bars + kBarFull + 8u * s, ((use + g) / kSlots) & 1u, kLimit);
+                                if (!ok) break;
+                            }
+#pragma unroll
+                            for (uint32_t j = 0; j < 4; ++j)
+                                mma(d, a + 32u * g + 8u * j, w + 2u * j, id_half, (g | j) ? 1u : 0u);
+                            if (l == 2 && t + 1u == nt) mma_commit(bars + kBarFree + 8u * s);
+                        }
+                        if (!ok) break;
+                        mma_commit(bars + kBarD + 8u * t);
+                    }
+                    if (l == 2) use += 4u;
+                }
+                if (ok && !fixed) {
+                    ok = mbar_wait(bars + kBarFixed, 0u, kLimit);
+                    fixed = ok;
+                }
+                // output layer, N = 16
+#pragma unroll 1
+                for (uint32_t t = 0; t < nt && ok; ++t) {
+                    ok = mbar_wait(bars + kBarAct + 8u * t, (3u * k + 2u) & 1u, kLimit);
+                    if (!ok) break;
+                    fence_after();
+#pragma unroll
+                    for (uint32_t i = 0; i < 16; ++i)
+                        mma(tmem + kColD + 128u * t, tmem + kColA + 128u * t + 8u * i, w3 + 128u * (i >> 2) + 2u * (i & 3u),
+                            id_out, i ? 1u : 0u);
+                    mma_commit(bars + kBarOut + 8u * t);
+                }
+            }
+            if (!ok) atomicOr(P.err, 1u);
+            // issued tensor-core work retires before the tensor memory is
+            // freed (bounded): one more commit, on the barrier whose only
+            // phase so far was the last layer's weights', after the copies
+            // that were not waited for
+            if (!fixed) {
+                for (uint32_t g = 0; g < 4; ++g) mbar_wait(bars + kBarW1 + 8u * g, 0u, kLimit);
+                mbar_wait(bars + kBarFixed, 0u, kLimit);
+            }
+            mma_commit(bars + kBarFixed);
+            if (!mbar_wait(bars + kBarFixed, 1u, kLimit)) atomicOr(P.err, 1u);
+        }
+        __syncwarp();
+    } else {
+        // ---- epilogue warps: block t = warp / 8, columns 64 sub .. +63 of each half
+        const uint32_t t = (uint32_t)warp >> 3, sub = ((uint32_t)warp >> 2) & 1u;
+        const uint32_t lanes = (32u * (uint32_t)(warp & 3)) << 16;
+        const uint32_t d = tmem + kColD + 128u * t + lanes + 64u * sub, a = tmem + kColA + 128u * t + lanes + 32u * sub;
+        uint32_t k = 0;
+#pragma unroll 1
+        for (uint32_t group = first; t < both && both * group + t < n_blocks && ok; group += stride, ++k) {
+#pragma unroll 1
+            for (uint32_t l = 0; l < 3; ++l) {
+                const float* b = bias + l * kHid + 64u * sub;
+                uint32_t z[32], w0[16], w1[16];
+                ok = mbar_wait(bars + kBarD + 8u * t, 0u, kLimit);   // six phases a group: halves alternate
+                if (!ok) break;
+                fence_after();
+                tmem_ld32(d, z);
+                silu32(z, b, w0);
+                tmem_ld32(d + 32u, z);
                 fence_before();
-                fence_async_smem();
-                mbar_arrive(barF);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bars + kBarDrained + 8u * t);
+                silu32(z, b + 32, w1);
+                ok = mbar_wait(bars + kBarD + 8u * t, 1u, kLimit);   // the A operand is free now
+                if (!ok) break;
+                fence_after();
+                tmem_st16(a, w0);
+                tmem_st16(a + 16u, w1);
+                tmem_ld32(d, z);
+                silu32(z, b + 128, w0);
+                tmem_ld32(d + 32u, z);
+                tmem_st16(a + 64u, w0);
+                silu32(z, b + 160, w1);
+                tmem_st16(a + 80u, w1);
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bars + kBarAct + 8u * t);
             }
         }
-        if (!ok && lane == 0) atomicOr(err, 1u);
+        if (!ok && lane == 0) atomicOr(P.err, 1u);
     }
     fence_before();
     __syncthreads();
@@ -539,23 +599,31 @@ cudaError_t launch_pack_sw128(const void* src, int rows, int K, int ld, int kpad
 
 size_t mlp_tc_image_bytes() { return tc::kImgBytes; }
 
-cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, const float* fistd,
-                          const void* wimg, const float* b0, const float* b1, const float* b2, const float* b3,
-                          float* out, unsigned* err, cudaStream_t s)
+static cudaError_t launch_mlp(MlpParams P, cudaStream_t s)
 {
-    if (n == 0) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(mlp_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)tc::kSmemBytes);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 1;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    const uint32_t blocks = (n + tc::kRows - 1) / tc::kRows;
-    const uint32_t grid = blocks < (uint32_t)sms ? blocks : (uint32_t)sms;   // one CTA per SM
-    mlp_tc_kernel<<<grid, tc::kThreads, tc::kSmemBytes, s>>>(feats, n, fmean, fistd,
-                                                            static_cast<const unsigned char*>(wimg), b0, b1, b2,
-                                                            b3, out, err);
+    // one CTA per SM; two blocks in flight where there are more than CTAs
+    const uint32_t blocks = (P.n + tc::kRows - 1) / tc::kRows;
+    const uint32_t per_net = std::max(1u, (uint32_t)sms / P.n_nets);
+    P.in_flight = blocks > per_net ? 2u : 1u;
+    const uint32_t groups = (blocks + P.in_flight - 1) / P.in_flight;
+    mlp_tc_kernel<<<std::min(groups, per_net) * P.n_nets, tc::kThreads, tc::kSmemBytes, s>>>(P);
     return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, const float* fistd,
+                          const void* wimg, const float* b0, const float* b1, const float* b2, const float* b3,
+                          float* out, unsigned* err, cudaStream_t s)
+{
+    if (n == 0) return cudaSuccess;
+    MlpParams P{feats, n, 1u, 1u, {}, err};
+    P.net[0] = MlpNet{fmean, fistd, static_cast<const unsigned char*>(wimg), {b0, b1, b2, b3}, out};
+    return launch_mlp(P, s);
 }
 
 }  // namespace sfh

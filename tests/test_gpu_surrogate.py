@@ -495,6 +495,31 @@ def test_fused_tensor_core_kernel_against_oracle_layers(hctx, n):
         assert float(np.median(rel)) <= 2.0 ** -10, (first, float(np.median(rel)))
 
 
+@pytest.mark.parametrize("blocks,extra", [(1, -127), (1, 0), (153, 0), (304, 37)])
+def test_fused_inference_with_several_blocks_per_cta(hctx, blocks, extra):
+    """CTAs that take a second, third or fourth 128-state block (one block
+    more than the SMs, two rounds, a ragged last block) give the bits that the
+    same rows give in pieces of at most 100 blocks, one per CTA."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = (sms + blocks) * 128 + extra
+    rng = np.random.default_rng(blocks)
+    sur = S.Surrogate(hctx, hidden=256, seed=9, batch=256)
+    feats = _dev(rng.normal(size=(n, S.N_FEAT)) * 1.5 + 0.5)
+    targ = _dev(rng.normal(size=(4096, S.N_OUT)) * 40.0 + 5.0)
+    sur.fit_normalisation(feats[:4096], targ)
+    tcw = sur.tc_weights()
+    got = torch.full((n + 128, 16), -3.0, device="cuda")
+    sur.infer_tc(feats, got, tcw)
+    want = torch.empty((n, 16), device="cuda")
+    for a in range(0, n, 12800):
+        piece = feats[a:a + 12800].contiguous()
+        sur.infer_tc(piece, want[a:a + 12800], tcw)
+    torch.cuda.synchronize()
+    assert int(tcw["err"].item()) == 0
+    assert torch.equal(got[:n], want)
+    assert torch.all(got[n:] == -3.0)
+
+
 def test_fused_tensor_core_kernel_against_oracle_output(hctx):
     """The whole network as the gated predictor runs it (trained weights, the
     target de-normalisation folded into the last layer) against
