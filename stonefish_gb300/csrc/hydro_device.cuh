@@ -239,64 +239,138 @@ __device__ __forceinline__ v3 xform(const float* M, float x, float y, float z)
 }
 
 // ------------------------------------------------------------- wave height
+// A lookup is inlined for every vertex and face centroid of a step on waves
+// and set its pace there: chains of dependent operations and branches.  Two
+// points are looked up together (two vertices, two faces), so that their
+// texels load together; the roundings to integers are additions with
+// directed rounding instead of conversions; one test sends the rare points
+// (beyond 2^21 grids, not a number, on the wrap) to the general form.  1024
+// torpedoes of 20,000 faces on a 1024 x 1024 grid: chunk kernel 382 us with
+// four branches and eight conversions per lookup and one vertex at a time,
+// 333 us now (12.2 -> 11.3 instructions per face, 49 -> 55% issue).
+
+// i = floor(t) for 0 <= t < 2^23 with its value as a float in *f
+__device__ __forceinline__ uint32_t trunc_index(float t, float* f)
+{
+    const float m = __fadd_rz(t, 8388608.f);
+    *f = m - 8388608.f;
+    return __float_as_uint(m) - 0x4B000000u;
+}
+
+// v - floor(v) for |v| < 2^22; like v - trunc(v), or 1 - |v - trunc(v)| where
+// that is negative, it rounds the exact difference once
+__device__ __forceinline__ float frac_floor(float v) { return v - (__fadd_rd(v, 12582912.f) - 12582912.f); }
+
 __device__ __forceinline__ float fracf_(float x) { return x - truncf(x); }
 
-// Texel offset j * N + i of the four bilinear taps, wrapped modulo N * N,
-// times the channel count plus the channel.  The grid holds fewer than 2^32
-// values (hydro_wave_grid_set), so 32 bits hold every offset, also the
-// j * N + i of a tap one texel past the last row before it wraps.
-__device__ __forceinline__ uint32_t texel_offset(uint32_t N, int j, int i, uint32_t C, uint32_t ch)
+__device__ __forceinline__ float frac_wide(float v)
 {
-    const uint32_t NN = N * N;
-    uint32_t l = (uint32_t)j * N + (uint32_t)i;
-    if (l >= NN) l -= NN;
-    return l * C + ch;
+    const float f = fracf_(v);
+    return f < 0.f ? 1.f - fabsf(f) : f;
 }
+
+// The four bilinear taps of a lookup: texel offsets j * N + i modulo N * N
+// (the grid holds fewer than 2^32 values, hydro_wave_grid_set) and weights.
+struct WaveTaps {
+    uint32_t l0, l1, l2, l3;
+    float alpha, beta;
+};
 
 // OpenGLRealOcean::ComputeInterpolatedWaveData (OpenGLRealOcean.cpp:282-319),
 // texel-centred periodic bilinear; the linear texel index wraps modulo N*N
-// where the reference would read texel N of a row.
-__device__ __forceinline__ float wave_interp(const OceanDev& o, float x, float y, uint32_t ch)
+// where the reference would read texel N of a row.  False, and offsets that
+// must not be used, where the point is too far away or not a number or an
+// index is N (a fraction rounded up to one); wave_taps_wide then gives them.
+__device__ __forceinline__ bool wave_taps(const OceanDev& o, float x, float y, WaveTaps& t)
 {
     const uint32_t N = o.wave_n;
-    const float Nf = (float)N;
-    const float half = o.wave_half;   // 0.5f / Nf, formed once on the host (IEEE division there too)
-    float i0f = fracf_(x - half);
-    float j0f = fracf_(y - half);
-    if (i0f < 0.f) i0f = 1.f - fabsf(i0f);
-    if (j0f < 0.f) j0f = 1.f - fabsf(j0f);
-    int i0 = (int)truncf(i0f * Nf);
-    int j0 = (int)truncf(j0f * Nf);
-    float i1f = fracf_(x + half);
-    float j1f = fracf_(y + half);
-    if (i1f < 0.f) i1f = 1.f - fabsf(i1f);
-    if (j1f < 0.f) j1f = 1.f - fabsf(j1f);
-    int i1 = (int)truncf(i1f * Nf);
-    int j1 = (int)truncf(j1f * Nf);
-    float alpha = fracf_(i0f * Nf);
-    float beta = fracf_(j0f * Nf);
-    const float* d = o.wave_data;
+    const float Nf = (float)N, half = o.wave_half;   // 0.5f / Nf, an IEEE division on the host
+    const float ti = frac_floor(x - half) * Nf, tj = frac_floor(y - half) * Nf;
+    float f;
+    const uint32_t i0 = trunc_index(ti, &f);
+    t.alpha = ti - f;
+    const uint32_t j0 = trunc_index(tj, &f);
+    t.beta = tj - f;
+    const uint32_t i1 = trunc_index(frac_floor(x + half) * Nf, &f), j1 = trunc_index(frac_floor(y + half) * Nf, &f);
+    t.l0 = j0 * N + i0;
+    t.l1 = j0 * N + i1;
+    t.l2 = j1 * N + i0;
+    t.l3 = j1 * N + i1;
+    return fabsf(x) < 0x1p21f && fabsf(y) < 0x1p21f && (i0 | i1 | j0 | j1) < N;
+}
+
+__device__ __forceinline__ void wave_taps_wide(const OceanDev& o, float x, float y, WaveTaps& t)
+{
+    const uint32_t N = o.wave_n, NN = N * N;
+    const float Nf = (float)N, half = o.wave_half;
+    const float ti = frac_wide(x - half) * Nf, tj = frac_wide(y - half) * Nf;
+    const uint32_t i0 = (uint32_t)(int)truncf(ti), j0 = (uint32_t)(int)truncf(tj);
+    const uint32_t i1 = (uint32_t)(int)truncf(frac_wide(x + half) * Nf);
+    const uint32_t j1 = (uint32_t)(int)truncf(frac_wide(y + half) * Nf);
+    t.alpha = fracf_(ti);
+    t.beta = fracf_(tj);
+    const uint32_t l0 = j0 * N + i0, l1 = j0 * N + i1, l2 = j1 * N + i0, l3 = j1 * N + i1;
+    t.l0 = l0 >= NN ? l0 - NN : l0;
+    t.l1 = l1 >= NN ? l1 - NN : l1;
+    t.l2 = l2 >= NN ? l2 - NN : l2;
+    t.l3 = l3 >= NN ? l3 - NN : l3;
+}
+
+__device__ __forceinline__ float wave_sample(const OceanDev& o, const WaveTaps& t, uint32_t ch)
+{
+    const float* d = o.wave_data + ch;
     const uint32_t C = o.wave_channels;
-    // 32-bit offsets: hydro_wave_grid_set keeps N * N * channels below 2^32
-    // (one code path at every inlined lookup keeps the kernels' instruction
-    // footprint small)
-    const float t0 = __ldg(d + texel_offset(N, j0, i0, C, ch));
-    const float t1 = __ldg(d + texel_offset(N, j0, i1, C, ch));
-    const float t2 = __ldg(d + texel_offset(N, j1, i0, C, ch));
-    const float t3 = __ldg(d + texel_offset(N, j1, i1, C, ch));
+    const float t0 = __ldg(d + t.l0 * C);
+    const float t1 = __ldg(d + t.l1 * C);
+    const float t2 = __ldg(d + t.l2 * C);
+    const float t3 = __ldg(d + t.l3 * C);
+    const float alpha = t.alpha, beta = t.beta;
     return (1.f - alpha) * (1.f - beta) * t0 + alpha * (1.f - beta) * t1
          + (1.f - alpha) * beta * t2 + alpha * beta * t3;
 }
 
-// OpenGLRealOcean::ComputeWaveHeight (:321-331).  x / gs is the IEEE
-// quotient, formed from RN(1 / gs) with one FMA correction (div_by_rcp).
+// x / gs, the IEEE quotient formed from RN(1 / gs) with one FMA correction
+// (div_by_rcp).  A numerator below 2^-100, for which that can miss the last
+// bit, is nothing beside the half texel that the lookup adds to it.
+__device__ __forceinline__ float grid_quotient(float x, float gs, float r)
+{
+    const float q = x * r;
+    return __fmaf_rn(__fmaf_rn(-gs, q, x), r, q);
+}
+
+// OpenGLRealOcean::ComputeWaveHeight (:321-331)
 __device__ __forceinline__ float wave_height(const OceanDev& o, float x, float y)
 {
     float z = 0.f;
     if (o.wave_data == nullptr) return z;
     for (uint32_t l = 0; l < o.wave_layers; ++l) {
         const float gs = o.wave_grid[l], r = o.wave_inv_grid[l];
-        z -= wave_interp(o, div_by_rcp(x, gs, r), div_by_rcp(y, gs, r), o.wave_channel[l]);
+        const float u = grid_quotient(x, gs, r), v = grid_quotient(y, gs, r);
+        WaveTaps t;
+        if (!wave_taps(o, u, v, t)) wave_taps_wide(o, u, v, t);
+        z -= wave_sample(o, t, o.wave_channel[l]);
+    }
+    return z;
+}
+
+// The heights at two points, with one test for both and their texels' loads
+// together in flight.
+__device__ __forceinline__ float2 wave_height2(const OceanDev& o, float2 x, float2 y)
+{
+    float2 z = make_float2(0.f, 0.f);
+    if (o.wave_data == nullptr) return z;
+    for (uint32_t l = 0; l < o.wave_layers; ++l) {
+        const float gs = o.wave_grid[l], r = o.wave_inv_grid[l];
+        const float ua = grid_quotient(x.x, gs, r), va = grid_quotient(y.x, gs, r);
+        const float ub = grid_quotient(x.y, gs, r), vb = grid_quotient(y.y, gs, r);
+        WaveTaps a, b;
+        const bool oka = wave_taps(o, ua, va, a), okb = wave_taps(o, ub, vb, b);
+        if (!(oka && okb)) {
+            wave_taps_wide(o, ua, va, a);
+            wave_taps_wide(o, ub, vb, b);
+        }
+        z.x -= wave_sample(o, a, o.wave_channel[l]);
+        z.y -= wave_sample(o, b, o.wave_channel[l]);
     }
     return z;
 }
@@ -420,6 +494,17 @@ __device__ __forceinline__ float depth_at_b(const OceanDev& o, const BodyParams&
     if (!o.waves) return z;
     if (B.centred) return z - wave_height(o, x + B.off[0], y + B.off[1]);
     return z - wave_height(o, x, y);
+}
+
+__device__ __forceinline__ float2 depth_at_b2(const OceanDev& o, const BodyParams& B, float2 x, float2 y, float2 z)
+{
+    if (!o.waves) return z;
+    if (B.centred) {
+        x = make_float2(x.x + B.off[0], x.y + B.off[0]);
+        y = make_float2(y.x + B.off[1], y.y + B.off[1]);
+    }
+    const float2 h = wave_height2(o, x, y);
+    return make_float2(z.x - h.x, z.y - h.y);
 }
 
 // FIELD = false: compiled for launches without jet or pipe currents (the

@@ -229,7 +229,7 @@ __device__ __forceinline__ void face_full2(const OceanDev& o, const BodyParams& 
     float2 A;
     tri_props2(p1, p2, p3, fc, fn1, A, validB);
     if (WAVES && B.buoyancy) {
-        float2 dc = f2(depth_at_b(o, B, fc.x.x, fc.y.x, fc.z.x), depth_at_b(o, B, fc.x.y, fc.y.y, fc.z.y));
+        const float2 dc = depth_at_b2(o, B, fc.x, fc.y, fc.z);
         P3 Fbi = pmul(pmul(pk(neg2(fn1.x), neg2(fn1.y), neg2(fn1.z)), A), dc);
         acc_add3p(a, Q_FB, Fbi);
         acc_add3p(a, Q_TB, pcross(psub(fc, Bp.p), Fbi));
