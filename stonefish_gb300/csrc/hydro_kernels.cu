@@ -876,11 +876,14 @@ __device__ __forceinline__ void transform_tile(const KParams& P, const StageBuf&
             under = !(d.x < 0.f) || !(d.y < 0.f);
         }
     } else {
-        for (int v = threadIdx.x; v < nv; v += kBlock) {
+        const int pairs = (nv + 1) >> 1, v = threadIdx.x, w = v + pairs < nv ? v + pairs : v;
+        if (v < pairs) {
             const v3 p = xform(TC, raw[v], raw[nvp + v], raw[2 * nvp + v]);
+            const v3 q = xform(TC, raw[w], raw[nvp + w], raw[2 * nvp + w]);
             out[v] = make_float4(p.x, p.y, p.z, p.z);
-            above |= p.z < 0.f;
-            under |= !(p.z < 0.f);
+            out[w] = make_float4(q.x, q.y, q.z, q.z);
+            above = p.z < 0.f || q.z < 0.f;
+            under = !(p.z < 0.f) || !(q.z < 0.f);
         }
     }
     const unsigned a = __ballot_sync(0xffffffffu, above), u = __ballot_sync(0xffffffffu, under);
