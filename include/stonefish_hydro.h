@@ -959,6 +959,63 @@ hydro_status hydro_nn_audit_error(hydro_ctx* ctx, const hydro_body* d_bodies, co
                                   uint32_t k, double force_scale, double torque_scale, float* d_err,
                                   void* stream);
 
+/* One network of a prediction: hydro_nn_mlp_tc's operands and its output
+ * rows [n][16]. */
+typedef struct hydro_nn_predict_net {
+    const float* fmean;
+    const float* fistd;
+    const void* image;
+    const float* bias[4];
+    float* z;
+} hydro_nn_predict_net;
+
+/* Gated prediction of n states (device pointers).  n_nets 1 or 2; the gate of
+ * hydro_nn_gate, with gate_inside that of hydro_nn_gate_inside; two networks
+ * give their mean and the gate of hydro_nn_ensemble at tau (infinity: off).
+ * audit_stride > 0 samples as hydro_nn_audit_pick does.  Work buffers:
+ * features [n][16], mask [n], counts [(n + 255) / 256], packed [n], pos [n],
+ * rows [n], n_packed [1], exact [n]; features, z and out 16-byte aligned.
+ * Every field is read at the call. */
+typedef struct hydro_nn_predictor {
+    uint32_t n;
+    int32_t n_nets;
+    int32_t gate_inside;
+    float threshold;
+    float tau;
+    uint32_t audit_stride;
+    uint32_t split_chunks;
+    uint32_t reserved;
+    double force_scale, torque_scale;
+    const float* lo;
+    const float* hi;
+    const float* mean;
+    const float* precision;
+    hydro_nn_predict_net net[2];
+    uint32_t* err;
+    float* features;
+    uint8_t* mask;
+    uint32_t* counts;
+    hydro_body* packed;
+    int32_t* pos;
+    uint32_t* rows;
+    uint32_t* n_packed;
+    hydro_wrench* exact;
+    float* out;
+} hydro_nn_predictor;
+
+/* out [n][6] = the networks' body-frame wrench for the states the gates admit
+ * and the exact step's for the others and the audit sample: the results of
+ * hydro_nn_features, _gate, _gate_inside, _mlp_tc, _ensemble, _audit_pick,
+ * _route, hydro_batch_compute_device_prefix, _merge and _audit_error in turn,
+ * in six launches (fourteen with two networks and the audit).  `batch` holds
+ * n bodies of one mesh.  With split_chunks the exact step's chunks are split
+ * into smaller ones while few states take it, which changes the order of its
+ * FP32 sums (not their accuracy) with the number of such states.  audit_err: one float per sample.
+ * *launches (optional) receives the kernels launched. */
+hydro_status hydro_nn_predict(hydro_ctx* ctx, hydro_batch* batch, const hydro_nn_predictor* p,
+                              const hydro_body* d_states, const hydro_ocean* ocean, const hydro_settings* settings,
+                              uint32_t audit_phase, float* d_audit_err, uint32_t* launches, void* stream);
+
 /* d_out[i][6] = body-frame wrench: columns 0..5 of d_z[i] (row stride ld)
  * when d_pos[i] < 0, else R^T (Fb+Fdq+Fdf, Tb+Tdq+Tdf) of d_exact[d_pos[i]]. */
 hydro_status hydro_nn_merge(hydro_ctx* ctx, const hydro_body* d_bodies, const float* d_z, int32_t ld,

@@ -144,6 +144,20 @@ class NnNet(C.Structure):
                 ("batch", C.c_int32), ("n_out", C.c_int32)]
 
 
+class NnPredictNet(C.Structure):
+    _fields_ = [("fmean", C.c_void_p), ("fistd", C.c_void_p), ("image", C.c_void_p), ("bias", C.c_void_p * 4),
+                ("z", C.c_void_p)]
+
+
+class NnPredictor(C.Structure):
+    _fields_ = [("n", C.c_uint32), ("n_nets", C.c_int32), ("gate_inside", C.c_int32), ("threshold", C.c_float),
+                ("tau", C.c_float), ("audit_stride", C.c_uint32), ("split_chunks", C.c_uint32), ("reserved", C.c_uint32),
+                ("force_scale", C.c_double), ("torque_scale", C.c_double), ("lo", C.c_void_p), ("hi", C.c_void_p), ("mean", C.c_void_p),
+                ("precision", C.c_void_p), ("net", NnPredictNet * 2), ("err", C.c_void_p), ("features", C.c_void_p),
+                ("mask", C.c_void_p), ("counts", C.c_void_p), ("packed", C.c_void_p), ("pos", C.c_void_p),
+                ("rows", C.c_void_p), ("n_packed", C.c_void_p), ("exact", C.c_void_p), ("out", C.c_void_p)]
+
+
 class TuneResult(C.Structure):
     _fields_ = [("chunk_faces", C.c_uint32), ("ctas_per_sm", C.c_uint32), ("ms_per_step", C.c_float),
                 ("from_cache", C.c_int32), ("n_candidates", C.c_uint32), ("candidate_ms", C.c_float * 16)]
@@ -272,6 +286,8 @@ def _declare(lib: C.CDLL) -> None:
                                  C.c_float, C.c_float, i32, vp, vp, vp]),
         "hydro_nn_train": (i32, [vp, C.POINTER(NnNet), vp, vp, C.c_int64, vp, vp, i32, i32, C.c_float, C.c_float,
                                  C.c_float, C.c_float, vp]),
+        "hydro_nn_predict": (i32, [vp, vp, C.POINTER(NnPredictor), vp, C.POINTER(Ocean), C.POINTER(Settings), u32, vp,
+                                   C.POINTER(u32), vp]),
         "hydro_nn_to_bf16": (i32, [vp, vp, i32, i32, i32, vp, vp, vp, vp]),
         "hydro_nn_features": (i32, [vp, vp, u32, C.POINTER(Ocean), vp, vp]),
         "hydro_nn_gate": (i32, [vp, vp, u32, vp, vp, vp, vp, C.c_float, vp, vp]),

@@ -411,15 +411,16 @@ hydro_status batch_build(hydro_ctx* ctx, const hydro_mesh_id* mesh_of_body, uint
     return HYDRO_OK;
 }
 
-hydro_status batch_launch(hydro_batch* b, const hydro_body* d_bodies, const hydro_ocean* ocean,
-                          const hydro_settings* settings, hydro_wrench* d_io, cudaStream_t s,
-                          int op, const uint32_t* d_count = nullptr, hydro_aero_wrench* d_aero = nullptr,
-                          const hydro_aero_params* d_aero_params = nullptr)
+// Kernel parameters and launch shape of a step of batch b.
+hydro_status batch_params(hydro_batch* b, const hydro_body* d_bodies, const hydro_ocean* ocean,
+                          const hydro_settings* settings, hydro_wrench* d_io, int op, const uint32_t* d_count,
+                          hydro_aero_wrench* d_aero, const hydro_aero_params* d_aero_params, KParams& P,
+                          LaunchShape& shape)
 {
     hydro_ctx* ctx = b->ctx;
     hydro_status st = sync_tiles(ctx);
     if (st != HYDRO_OK) return st;
-    KParams P{};
+    P = KParams{};
     P.chunks = b->chunks_d;
     P.binfo = b->binfo_d;
     P.tiles = ctx->tiles_d;
@@ -445,12 +446,26 @@ hydro_status batch_launch(hydro_batch* b, const hydro_body* d_bodies, const hydr
     if (P.ocean.waves && ctx->wave_d == nullptr)
         return fail(ctx, HYDRO_ERR_INVALID_ARG, "ocean.waves set but no wave grid was given");
     const int cut64 = ctx->cfg.cut_precision == HYDRO_CUT_FP64;
-    LaunchShape shape{};
+    shape = LaunchShape{};
     const int want = b->ctas_per_sm ? (int)b->ctas_per_sm : ctx->cfg.ctas_per_sm ? (int)ctx->cfg.ctas_per_sm : 2;
     shape.ctas_per_sm = std::max(1, std::min(want, chunk_kernel_occupancy(cut64, P.ocean.waves, want,
                                                                             op == OP_AERO || op == OP_AERO_BODY,
                                                                             P.ocean.field_currents)));
     shape.grid = ctx->sm_count * shape.ctas_per_sm;
+    return HYDRO_OK;
+}
+
+hydro_status batch_launch(hydro_batch* b, const hydro_body* d_bodies, const hydro_ocean* ocean,
+                          const hydro_settings* settings, hydro_wrench* d_io, cudaStream_t s,
+                          int op, const uint32_t* d_count = nullptr, hydro_aero_wrench* d_aero = nullptr,
+                          const hydro_aero_params* d_aero_params = nullptr)
+{
+    hydro_ctx* ctx = b->ctx;
+    KParams P;
+    LaunchShape shape;
+    const hydro_status st = batch_params(b, d_bodies, ocean, settings, d_io, op, d_count, d_aero, d_aero_params, P, shape);
+    if (st != HYDRO_OK) return st;
+    const int cut64 = ctx->cfg.cut_precision == HYDRO_CUT_FP64;
     uint32_t launches = 0;
     // kernel timing events (hydro_batch_profile) outside stream capture only
     cudaEvent_t* ev = nullptr;
@@ -2396,6 +2411,57 @@ extern "C" hydro_status hydro_nn_audit_error(hydro_ctx* ctx, const hydro_body* d
     NN_RET(launch_audit_error(d_bodies, d_z, ld, d_pos, d_exact, d_idx, k, (float)(1.0 / force_scale),
                               (float)(1.0 / torque_scale), d_err, static_cast<cudaStream_t>(stream)),
            "nn audit error");
+}
+
+extern "C" hydro_status hydro_nn_predict(hydro_ctx* ctx, hydro_batch* batch, const hydro_nn_predictor* p,
+                                         const hydro_body* d_states, const hydro_ocean* ocean,
+                                         const hydro_settings* settings, uint32_t audit_phase, float* d_audit_err,
+                                         uint32_t* launches, void* stream)
+{
+    NN_CTX_CHECK();
+    if (!batch || batch->ctx != ctx || !p || !d_states || !settings || !valid_ocean(ocean) || p->n_nets < 1 || p->n_nets > 2)
+        return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: missing argument");
+    const hydro_nn_predictor& q = *p;
+    if (q.n == 0 || q.n != batch->n_bodies || q.n >= kAuditedRow || !q.lo || !q.hi || !q.mean || !q.precision || !q.err || !q.features || !q.mask ||
+        !q.counts || !q.packed || !q.pos || !q.rows || !q.n_packed || !q.exact || !q.out || !(q.force_scale > 0.0) ||
+        !(q.torque_scale > 0.0) || (q.audit_stride && (!d_audit_err || audit_phase >= q.audit_stride)))
+        return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: bad predictor");
+    uintptr_t align = reinterpret_cast<uintptr_t>(q.features) | reinterpret_cast<uintptr_t>(q.out);
+    for (int k = 0; k < q.n_nets; ++k) {
+        const hydro_nn_predict_net& N = q.net[k];
+        if (!N.fmean || !N.fistd || !N.image || !N.bias[0] || !N.bias[1] || !N.bias[2] || !N.bias[3] || !N.z)
+            return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: bad network");
+        align |= reinterpret_cast<uintptr_t>(N.image) | reinterpret_cast<uintptr_t>(N.z);
+    }
+    if (align & 15) return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: buffers must be 16-byte aligned");
+    for (uint32_t m : batch->mesh_of_body)
+        if (m != batch->mesh_of_body[0]) return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: the batch needs one mesh");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    KParams P;
+    LaunchShape shape;
+    const hydro_status st = batch_params(batch, q.packed, ocean, settings, q.exact, OP_BODY, q.n_packed, nullptr, nullptr, P,
+                                         shape);
+    if (st != HYDRO_OK) return st;
+    P.split_tiles = q.split_chunks ? batch->chunk_tiles : 0u;
+    P.split_grid = (uint32_t)shape.grid;
+    const float inv_fs = (float)(1.0 / q.force_scale), inv_ts = (float)(1.0 / q.torque_scale);
+    P.merge = KParams::Merge{q.rows, q.out, q.net[0].z, d_audit_err, q.audit_stride, audit_phase, inv_fs, inv_ts};
+    PredictNet nets[2] = {};
+    for (int k = 0; k < q.n_nets; ++k) {
+        const hydro_nn_predict_net& N = q.net[k];
+        nets[k] = PredictNet{N.fmean, N.fistd, N.image, {N.bias[0], N.bias[1], N.bias[2], N.bias[3]}, N.z};
+    }
+    const GateParams g{q.lo, q.hi, q.mean, q.precision, q.threshold, q.gate_inside};
+    cudaError_t e = launch_states(d_states, q.n, P.ocean, g, q.features, q.mask, s);
+    if (e == cudaSuccess) e = launch_mlp_nets(q.features, q.n, nets, q.n_nets, q.err, s);
+    if (e == cudaSuccess)
+        e = launch_combine(q.net[0].z, q.n_nets > 1 ? q.net[1].z : nullptr, q.n, inv_fs, inv_ts, q.tau, q.audit_stride,
+                           audit_phase, d_audit_err, q.mask, q.counts, q.out, s);
+    if (e == cudaSuccess)
+        e = launch_predict_step(P, d_states, q.mask, q.n, q.counts, q.packed, q.pos, q.rows, q.n_packed, shape,
+                                ctx->cfg.cut_precision == HYDRO_CUT_FP64, s);
+    if (launches) *launches = 6u;
+    NN_RET(e, "nn predict");
 }
 
 // ====================================================== rigid-body rollout

@@ -382,6 +382,44 @@ __device__ __forceinline__ float depth_at(const OceanDev& o, float x, float y, f
     return z;
 }
 
+// The same at two points.
+__device__ __forceinline__ float2 depth_at2(const OceanDev& o, float2 x, float2 y, float2 z)
+{
+    if (!o.waves) return z;
+    const float2 h = wave_height2(o, x, y);
+    return make_float2(z.x - h.x, z.y - h.y);
+}
+
+// SolidEntity::CheckBodyFluidPosition with Ocean::GetDepth(const Vector3&):
+// each AABB corner cast to float, depth compared > 0 in double.  Two corners
+// at a time.
+__device__ __forceinline__ int classify(const OceanDev& o, const double* mn, const double* mx)
+{
+    const double d0 = mx[0] - mn[0], d1 = mx[1] - mn[1], d2 = mx[2] - mn[2];
+    const double c[8][3] = {
+        {mn[0], mn[1], mn[2]},
+        {mx[0], mx[1], mx[2]},
+        {mn[0] + d0, mn[1] + 0.0, mn[2] + 0.0},
+        {mn[0] + 0.0, mn[1] + d1, mn[2] + 0.0},
+        {mn[0] + d0, mn[1] + d1, mn[2] + 0.0},
+        {mn[0] + 0.0, mn[1] + 0.0, mn[2] + d2},
+        {mn[0] + d0, mn[1] + 0.0, mn[2] + d2},
+        {mn[0] + 0.0, mn[1] + d1, mn[2] + d2},
+    };
+    unsigned under = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        const float2 dep = depth_at2(o, make_float2((float)c[k][0], (float)c[k + 1][0]),
+                                     make_float2((float)c[k][1], (float)c[k + 1][1]),
+                                     make_float2((float)c[k][2], (float)c[k + 1][2]));
+        if (dep.x > 0.f) ++under;
+        if (dep.y > 0.f) ++under;
+    }
+    if (under == 0) return HYDRO_OUTSIDE;
+    if (under == 8) return HYDRO_INSIDE;
+    return HYDRO_CROSSING_SURFACE;
+}
+
 // ---------------------------------------------------------------- currents
 __device__ __forceinline__ double bdot(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 __device__ __forceinline__ void bcross(const double* a, const double* b, double* r)

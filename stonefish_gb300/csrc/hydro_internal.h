@@ -33,7 +33,39 @@ struct KParams {
     // largest first: class c (chunks of kMaxTilesPerChunk - 2c or one tile
     // fewer) owns active[class_start[c], class_start[c + 1]).
     uint32_t class_start[kClaimClasses + 1];
+    // Chunks split into parts when a device count leaves few bodies active
+    // (split_factor): tiles per chunk and CTAs of the chunk kernel, or zero.
+    uint32_t split_tiles;
+    uint32_t split_grid;
+    // Gated prediction: each evaluated body's body-frame wrench goes to its
+    // state's row of merge.out as well (null: not a prediction).
+    struct Merge {
+        const uint32_t* rows;    // packed slot -> state, kAuditedRow set for audited states
+        float* out;              // [n][6]
+        const float* z;          // network outputs, rows of 16
+        float* audit_err;        // per audit sample
+        uint32_t audit_stride, audit_phase;
+        float inv_fs, inv_ts;
+    } merge;
 };
+
+constexpr uint32_t kAuditedRow = 0x80000000u;
+
+// Parts per chunk of a step that evaluates the first n_active bodies of a
+// batch with one mesh: one while there are two chunks per CTA, else as many
+// as give that, down to parts of one tile, as far as the partial sums' room
+// (one slot per chunk of the batch) goes.
+__host__ __device__ inline uint32_t split_factor(uint32_t split_tiles, uint32_t split_grid, uint32_t n_active,
+                                                 uint32_t n_bodies, uint32_t n_chunks)
+{
+    if (split_tiles == 0u || n_active == 0u || n_active >= n_bodies) return 1u;
+    const uint32_t chunks = n_active * (n_chunks / n_bodies);
+    uint32_t f = 2u * split_grid / chunks;
+    const uint32_t room = n_bodies / n_active;
+    f = f < room ? f : room;
+    f = f < split_tiles ? f : split_tiles;
+    return f > 1u ? f : 1u;
+}
 
 // Claim class of a chunk of n_tiles tiles (largest chunks first), and the
 // class regions of a work list (exclusive prefix sums of the class sizes).
@@ -174,6 +206,38 @@ cudaError_t launch_rigid_write_bodies(const hydro_rigid_state* states, hydro_bod
 
 cudaError_t launch_pack_sw128(const void* src, int rows, int K, int ld, int kpad, void* dst, cudaStream_t s);
 size_t mlp_tc_image_bytes();
+
+// One network of a gated prediction, as launch_mlp_tc takes it.
+struct PredictNet {
+    const float* fmean;
+    const float* fistd;
+    const void* image;
+    const float* b[4];
+    float* z;            // outputs, rows of 16
+};
+cudaError_t launch_mlp_nets(const float* feats, uint32_t n, const PredictNet* nets, int n_nets, unsigned* err,
+                            cudaStream_t s);
+
+// Features, gate and (inside) the INSIDE test of every state in one pass.
+struct GateParams {
+    const float *lo, *hi, *mean, *P;
+    float thresh;
+    int inside;
+};
+cudaError_t launch_states(const hydro_body* bodies, uint32_t n, OceanDev o, const GateParams& g, float* feats,
+                          uint8_t* mask, cudaStream_t s);
+// Mean of the networks' outputs (into z0), disagreement gate, audit sample,
+// outputs of the admitted states, rejects per block of kCombineBlock states.
+// mask: 1 admitted, 0 rejected, 2 audited.
+constexpr int kCombineBlock = 256;
+cudaError_t launch_combine(float* z0, const float* z1, uint32_t n, float inv_fs, float inv_ts, float tau,
+                           uint32_t audit_stride, uint32_t audit_phase, float* audit_err, uint8_t* mask,
+                           uint32_t* counts, float* out, cudaStream_t s);
+// The exact step for the rejected states: packed in index order (with the
+// per-body preparation), chunk kernel, finalisation with the merge of P.
+cudaError_t launch_predict_step(const KParams& P, const hydro_body* states, uint8_t* mask, uint32_t n,
+                                const uint32_t* counts, hydro_body* packed, int32_t* pos, uint32_t* rows,
+                                uint32_t* n_packed, LaunchShape shape, int cut64, cudaStream_t s);
 cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, const float* fistd,
                           const void* wimg, const float* b0, const float* b1, const float* b2, const float* b3,
                           float* out, unsigned* err, cudaStream_t s);

@@ -37,31 +37,6 @@ namespace sfh {
 // --------------------------------------------------------------- FP64 helpers
 struct d3 { double x, y, z; };
 
-// SolidEntity::CheckBodyFluidPosition with Ocean::GetDepth(const Vector3&):
-// each AABB corner cast to float, depth compared > 0 in double.
-__device__ int classify(const OceanDev& o, const double* mn, const double* mx)
-{
-    const double d0 = mx[0] - mn[0], d1 = mx[1] - mn[1], d2 = mx[2] - mn[2];
-    const double c[8][3] = {
-        {mn[0], mn[1], mn[2]},
-        {mx[0], mx[1], mx[2]},
-        {mn[0] + d0, mn[1] + 0.0, mn[2] + 0.0},
-        {mn[0] + 0.0, mn[1] + d1, mn[2] + 0.0},
-        {mn[0] + d0, mn[1] + d1, mn[2] + 0.0},
-        {mn[0] + 0.0, mn[1] + 0.0, mn[2] + d2},
-        {mn[0] + d0, mn[1] + 0.0, mn[2] + d2},
-        {mn[0] + 0.0, mn[1] + d1, mn[2] + d2},
-    };
-    unsigned under = 0;
-    for (int k = 0; k < 8; ++k) {
-        float dep = depth_at(o, (float)c[k][0], (float)c[k][1], (float)c[k][2]);
-        if ((double)dep > 0.0) ++under;
-    }
-    if (under == 0) return HYDRO_OUTSIDE;
-    if (under == 8) return HYDRO_INSIDE;
-    return HYDRO_CROSSING_SURFACE;
-}
-
 // btMatrix3x3::inverse (3rdparty/LinearMath/btMatrix3x3.h:1093-1103)
 __device__ void binverse(const double* m, double* r)
 {
@@ -582,6 +557,43 @@ __device__ __forceinline__ void prefetch_lines(const void* p, size_t bytes, int 
 // except its last: the warp's full chunks take one run of their class (one
 // atomic, runs prefix-summed with shuffles, descriptors formed from the
 // body's first chunk), the last chunks one atomic per class present.
+// Lists a body's chunks cut into parts of `part` tiles (f parts per chunk at
+// most; part q of chunk c keeps its sums in slot c * f + q).  Called by all 32
+// lanes of a warp for a batch with one mesh, where every body has the same
+// chunks.
+__device__ __forceinline__ void list_parts(const KParams& P, uint32_t body, const BodyInfo& bi, uint32_t n, uint32_t f)
+{
+    const unsigned lane = threadIdx.x & 31u;
+    const uint32_t part = (P.split_tiles + f - 1u) / f;
+    uint4* act = reinterpret_cast<uint4*>(P.active);
+    // a full chunk and a last chunk in turn: their counts may be of two classes
+    for (int last = 0; last < 2; ++last) {
+        const uint32_t first = last ? n - 1u : 0u, count = n == 0u ? 0u : last ? 1u : n - 1u;
+        const uint4 d = count ? __ldg(reinterpret_cast<const uint4*>(P.chunks + bi.first_chunk) + first)
+                              : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t parts = (d.z + part - 1u) / part, cnt = count * parts;
+        const unsigned with = __ballot_sync(0xffffffffu, cnt > 0u);
+        if (with == 0u) continue;
+        const int leader = __ffs(with) - 1;
+        const uint32_t cls = __shfl_sync(0xffffffffu, claim_class(d.z), leader);
+        uint32_t incl = cnt;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, k);
+            if ((int)lane >= k) incl += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        uint32_t base = 0;
+        if ((int)lane == leader) base = atomicAdd(P.n_listed + cls, total);
+        base = P.class_start[cls] + __shfl_sync(0xffffffffu, base, leader) + incl - cnt;
+        for (uint32_t e = 0; e < cnt; ++e) {
+            const uint32_t j = e / parts, q = e - j * parts;
+            act[base + e] = make_uint4(body, d.y + j * d.z + q * part, min(part, d.z - q * part),
+                                       (bi.first_chunk + first + j) * f + q);
+        }
+    }
+}
+
 __device__ __forceinline__ void list_chunks(const KParams& P, uint32_t body, const BodyInfo& bi, uint32_t n)
 {
     const unsigned lane = threadIdx.x & 31u;
@@ -1170,6 +1182,33 @@ __global__ void __launch_bounds__(kThreads) __maxnreg__(MINB == 2 ? 128 : 255) c
     consumer<CUT64, WAVES, AERO, FIELD>(P, S);
 }
 
+// Total wrench in the body frame of an evaluated state (sub 0 its force, sub 1
+// its torque) into its row of the prediction, and, for an audited state, the
+// networks' error there (hydro_nn_audit_error's metric).
+__device__ __forceinline__ void merge_body(const KParams& P, uint32_t body, int sub)
+{
+    const uint32_t tag = P.merge.rows[body], row = tag & ~kAuditedRow;
+    const double* R = P.bodies[body].T_CG.basis;
+    const hydro_wrench& x = P.io[body];
+    double F[3], e2 = 0.0;
+    for (int k = 0; k < 3; ++k) F[k] = sub ? x.Tb[k] + x.Tdq[k] + x.Tdf[k] : x.Fb[k] + x.Fdq[k] + x.Fdf[k];
+    for (int k = 0; k < 3; ++k) {
+        const double f = R[k] * F[0] + R[3 + k] * F[1] + R[6 + k] * F[2];
+        P.merge.out[(size_t)row * 6 + 3 * sub + k] = (float)f;
+        if (tag & kAuditedRow) {
+            const double e = (double)P.merge.z[(size_t)row * 16 + 3 * sub + k] - f;
+            e2 += e * e;
+        }
+    }
+    if (tag & kAuditedRow) {   // both lanes of a body take this branch
+        const unsigned lane = threadIdx.x & 31u;
+        const double t2 = __shfl_down_sync(3u << (lane & ~1u), e2, 1);
+        if (sub == 0)
+            P.merge.audit_err[(row - P.merge.audit_phase) / P.merge.audit_stride] =
+                (float)fmax(sqrt(e2) * (double)P.merge.inv_fs, sqrt(t2) * (double)P.merge.inv_ts);
+    }
+}
+
 // ----------------------------------------------------------- finalise kernel
 // Four threads per body.  GB300 executes FP64 at about two lanes per clock
 // per SM and the finalisation is a chain of dependent FP64 operations, so
@@ -1190,6 +1229,7 @@ __global__ void __launch_bounds__(kBodyThreads) finalize_kernel(const KParams P)
     if (blockIdx.x == 0 && threadIdx.x < (unsigned)kClaimClasses)
         P.n_listed[threadIdx.x] = 0u;   // the chunk kernel has finished with them
     const uint32_t limit = P.n_active ? min(P.n_bodies, *P.n_active) : P.n_bodies;
+    const uint32_t split = split_factor(P.split_tiles, P.split_grid, limit, P.n_bodies, P.n_chunks);
     // grid-stride over groups of kPerCta bodies (uniform across the warp)
     for (uint32_t base = blockIdx.x * kPerCta; base < limit; base += gridDim.x * kPerCta) {
         const uint32_t body = base + (uint32_t)slot;
@@ -1215,7 +1255,20 @@ __global__ void __launch_bounds__(kBodyThreads) finalize_kernel(const KParams P)
             double s[kPer];
 #pragma unroll
             for (int i = 0; i < kPer; ++i) s[i] = 0.0;
-            if (B.loop != LOOP_NONE) {
+            if (B.loop != LOOP_NONE && split > 1u) {
+                // parts of chunks: the same order, several slots a chunk
+                const uint32_t part = (P.split_tiles + split - 1u) / split;
+                for (uint32_t c = 0; c < bi.n_chunks; ++c) {
+                    const uint32_t parts = (P.chunks[bi.first_chunk + c].n_tiles + part - 1u) / part;
+                    const double* p = P.partials + (size_t)(bi.first_chunk + c) * split * kPartialStride + sub;
+#pragma unroll 2
+                    for (uint32_t q = 0; q < parts; ++q, p += kPartialStride) {
+#pragma unroll
+                        for (int i = 0; i < kPer; ++i)
+                            if (sub + kFinSub * i < kQ) s[i] += p[kFinSub * i];
+                    }
+                }
+            } else if (B.loop != LOOP_NONE) {
                 const double* p = P.partials + (size_t)bi.first_chunk * kPartialStride + sub;
 #pragma unroll 2
                 for (uint32_t c = 0; c < bi.n_chunks; ++c, p += kPartialStride) {
@@ -1245,7 +1298,89 @@ __global__ void __launch_bounds__(kBodyThreads) finalize_kernel(const KParams P)
             double* dst = sub == 0 ? w.Fdq : sub == 1 ? w.Tdq : sub == 2 ? w.Fdf : w.Tdf;
             copy3(dst, v);
         }
-        __syncwarp();                  // sums are reused by the next group
+        __syncwarp();                  // sums are reused by the next group; the records are written
+        if (P.merge.out && live && sub < 2) merge_body(P, body, sub);
+    }
+}
+
+// Packs the rejected states (mask not 1) of a block of kCombineBlock in index
+// order, a warp copying a record, and prepares them as prep_kernel does:
+// slot order and results do not depend on scheduling.
+__global__ void __launch_bounds__(kCombineBlock)
+predict_pack_kernel(const KParams P, const hydro_body* __restrict__ states, uint8_t* __restrict__ mask, uint32_t n,
+                    const uint32_t* __restrict__ counts, uint32_t n_blocks, hydro_body* __restrict__ packed,
+                    int32_t* __restrict__ pos, uint32_t* __restrict__ rows, uint32_t* __restrict__ n_packed)
+{
+    __shared__ uint32_t warp_count[kCombineBlock / 32];
+    __shared__ uint32_t sums[2];
+    __shared__ uint32_t list[kCombineBlock];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {   // rejects before this block, and in all
+        uint32_t before = 0, total = 0;
+        for (uint32_t k = lane; k < n_blocks; k += 32) {
+            const uint32_t c = counts[k];
+            total += c;
+            if (k < blockIdx.x) before += c;
+        }
+        for (int o = 16; o; o >>= 1) {
+            before += __shfl_xor_sync(0xffffffffu, before, o);
+            total += __shfl_xor_sync(0xffffffffu, total, o);
+        }
+        if (lane == 0) {
+            sums[0] = before;
+            sums[1] = total;
+        }
+    }
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) *P.err = 0u;
+        if (threadIdx.x < (unsigned)kClaimClasses) P.work[threadIdx.x] = 0u;
+    }
+    const uint32_t i = blockIdx.x * kCombineBlock + threadIdx.x;
+    const uint8_t m = i < n ? mask[i] : (uint8_t)1;
+    const bool out = m != 1;
+    const unsigned bal = __ballot_sync(0xffffffffu, out);
+    if (lane == 0) warp_count[warp] = __popc(bal);
+    __syncthreads();
+    uint32_t rank = __popc(bal & ((1u << lane) - 1u)), mine = 0;
+    for (int w = 0; w < kCombineBlock / 32; ++w) {
+        if (w < warp) rank += warp_count[w];
+        mine += warp_count[w];
+    }
+    const uint32_t base = sums[0], total = sums[1];
+    if (i < n) {
+        pos[i] = out ? (int32_t)(base + rank) : -1;
+        if (out) {
+            list[rank] = i;
+            rows[base + rank] = i | (m == 2 ? kAuditedRow : 0u);
+            if (m == 2) mask[i] = 0;
+        }
+    }
+    if (i == 0) *n_packed = total;
+    __syncthreads();
+    constexpr uint32_t kWords = sizeof(hydro_body) / 8, kIoWords = sizeof(hydro_wrench) / 8;
+    for (uint32_t r = warp; r < mine; r += kCombineBlock / 32) {
+        const double* src = reinterpret_cast<const double*>(states + list[r]);
+        double* dst = reinterpret_cast<double*>(packed + base + r);
+        for (uint32_t k = lane; k < kWords; k += 32) dst[k] = src[k];
+        uint64_t* io = reinterpret_cast<uint64_t*>(P.io + base + r);   // fresh in-out record
+        if ((uint32_t)lane < kIoWords) io[lane] = 0ull;
+    }
+    static_assert(kIoWords <= 32, "one word per lane");
+    __syncthreads();
+    const uint32_t split = split_factor(P.split_tiles, P.split_grid, total, P.n_bodies, P.n_chunks);
+    if (32u * (uint32_t)warp < mine) {   // whole warps, for list_chunks
+        const uint32_t b = base + threadIdx.x;
+        BodyInfo bi{};
+        uint32_t c = 0;
+        if (threadIdx.x < mine) {
+            BodyParams B;
+            bi = P.binfo[b];
+            body_prologue(packed + b, bi.mesh, P.op, P.ocean, P.st, P.frame, B);
+            P.bparams[b] = B;
+            c = B.loop != LOOP_NONE ? bi.n_chunks : 0u;
+        }
+        if (split > 1u) list_parts(P, b, bi, c, split);
+        else list_chunks(P, b, bi, c);
     }
 }
 
@@ -1314,21 +1449,17 @@ int chunk_kernel_occupancy(int cut64, int waves, int ctas_per_sm, int aero, int 
     return n;
 }
 
-cudaError_t launch_step(const KParams& P, LaunchShape shape, int cut64, cudaStream_t s,
-                        uint32_t* launches, cudaEvent_t* ev)
+// Per-body kernels run at most eight warp-sized CTAs per SM, grid-stride
+// beyond (a device count may leave most of a large batch idle).
+static uint32_t body_cap(LaunchShape shape) { return 8u * (uint32_t)std::max(1, shape.grid / std::max(1, shape.ctas_per_sm)); }
+
+// The chunk kernel and the finalisation of prepared bodies.
+static cudaError_t launch_chunks(const KParams& P, LaunchShape shape, int cut64, cudaStream_t s, cudaEvent_t* ev)
 {
-    *launches = 0;
-    if (P.n_bodies == 0) return cudaSuccess;
     cudaError_t e;
-    if (ev && (e = cudaEventRecord(ev[0], s))) return e;
-    // per-body kernels: at most eight warp-sized CTAs per SM, grid-stride
-    // beyond (a device count may leave most of a large batch idle)
-    const uint32_t cap = 8u * (uint32_t)std::max(1, shape.grid / std::max(1, shape.ctas_per_sm));
-    prep_kernel<<<std::min((P.n_bodies + kBodyThreads - 1) / kBodyThreads, cap), kBodyThreads, 0, s>>>(P);
-    if ((e = cudaGetLastError())) return e;
-    if (ev && (e = cudaEventRecord(ev[1], s))) return e;
+    const uint32_t cap = body_cap(shape);
     int grid = shape.grid;
-    if (grid > (int)P.n_chunks) grid = (int)P.n_chunks;
+    if (grid > (int)P.n_chunks && P.split_tiles == 0u) grid = (int)P.n_chunks;
     if (grid < 1) grid = 1;
     const int aero = (P.op == OP_AERO || P.op == OP_AERO_BODY) ? 1 : 0;
     const int field = P.ocean.field_currents ? 1 : 0;
@@ -1341,8 +1472,34 @@ cudaError_t launch_step(const KParams& P, LaunchShape shape, int cut64, cudaStre
                       kBodyThreads, 0, s>>>(P);
     if ((e = cudaGetLastError())) return e;
     if (ev && (e = cudaEventRecord(ev[3], s))) return e;
+    return cudaSuccess;
+}
+
+cudaError_t launch_step(const KParams& P, LaunchShape shape, int cut64, cudaStream_t s,
+                        uint32_t* launches, cudaEvent_t* ev)
+{
+    *launches = 0;
+    if (P.n_bodies == 0) return cudaSuccess;
+    cudaError_t e;
+    if (ev && (e = cudaEventRecord(ev[0], s))) return e;
+    const uint32_t cap = body_cap(shape);
+    prep_kernel<<<std::min((P.n_bodies + kBodyThreads - 1) / kBodyThreads, cap), kBodyThreads, 0, s>>>(P);
+    if ((e = cudaGetLastError())) return e;
+    if (ev && (e = cudaEventRecord(ev[1], s))) return e;
+    if ((e = launch_chunks(P, shape, cut64, s, ev))) return e;
     *launches = 3;
     return cudaSuccess;
+}
+
+cudaError_t launch_predict_step(const KParams& P, const hydro_body* states, uint8_t* mask, uint32_t n,
+                                const uint32_t* counts, hydro_body* packed, int32_t* pos, uint32_t* rows,
+                                uint32_t* n_packed, LaunchShape shape, int cut64, cudaStream_t s)
+{
+    const uint32_t nb = (n + kCombineBlock - 1) / kCombineBlock;
+    predict_pack_kernel<<<nb, kCombineBlock, 0, s>>>(P, states, mask, n, counts, nb, packed, pos, rows, n_packed);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_chunks(P, shape, cut64, s, nullptr);
 }
 
 // ------------------------------------------------------------- compounds

@@ -33,12 +33,15 @@
 // Bound: MUFU (2,048 cycles per block and hidden layer) and the tensor pipe
 // (2,112), each with its hand-over: half a layer takes 1,450 cycles of either.
 // 65,536 states: 36.8 us with one block in flight and its activations in
-// shared memory, 26.7 us now (671 TFLOP/s, 34% of the measured 1,954).
+// shared memory, 28 us now (26.1 in a graph: 686 TFLOP/s, 35% of the measured
+// 1,954).  With no more blocks than CTAs a CTA takes one, its halves in an
+// accumulator each: 16,384 states 10.5 -> 9.8 us in a graph.
 //
 // Every mbarrier wait is bounded (%globaltimer); a timeout sets *err, the
 // CTA stops issuing work, waits (bounded) for its tensor-core work and its
 // copies to retire, frees its tensor memory and returns.
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -288,14 +291,14 @@ struct MlpParams {
     const float* feats;
     uint32_t n;
     uint32_t n_nets;
-    uint32_t in_flight;   // blocks per CTA at a time, 1 or 2
     MlpNet net[2];
     unsigned* err;
 };
 
-// CTA c works for network c % n_nets on the groups of in_flight 128-state
+// CTA c works for network c % n_nets on the groups of `both` 128-state
 // blocks c / n_nets, + gridDim.x / n_nets, ...  (the grid is a multiple of
 // n_nets).
+template <uint32_t both>
 __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_constant__ MlpParams P)
 {
     using namespace tc;
@@ -307,32 +310,57 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + kOffTmem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const MlpNet& N = P.net[blockIdx.x % P.n_nets];
-    const uint32_t n_blocks = (P.n + kRows - 1) / kRows, both = P.in_flight;
+    const uint32_t n_blocks = (P.n + kRows - 1) / kRows;
     const uint32_t n_groups = (n_blocks + both - 1) / both;
     const uint32_t first = blockIdx.x / P.n_nets, stride = gridDim.x / P.n_nets;
     const uint64_t kLimit = 1000000000ull;   // 1 s per wait
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 0) {
-        for (uint32_t b = 0; b < kBarEnd; b += 8) {
-            const uint32_t count = b >= kBarDrained && b < kBarIn ? 8u : b >= kBarIn && b < kBarW1 ? 4u : 1u;
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bars + b), "r"(count) : "memory");
+    // Before the CTA's first barrier, each role starts what takes longest: the
+    // weight copies, the feature loads, the tensor-memory allocation.
+    uint32_t copied = 0;   // weight slots filled (the copy warp's elected lane)
+    float raw_in[kIn];     // the first block's features (in/out warps, one block)
+    if (warp == kEpiWarps + 1) {
+        if (elect_one()) {
+            for (uint32_t b = 0; b < kBarEnd; b += 8) {
+                const uint32_t count = b >= kBarDrained && b < kBarIn ? 8u : b >= kBarIn && b < kBarW1 ? 4u : 1u;
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bars + b), "r"(count) : "memory");
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            for (; copied < 2; ++copied) {
+                expect_tx(bars + kBarFull + 8u * copied, 16384u);
+                bulk_load(sb + kOffRing + 16384u * copied, N.wimg + kImgW0 + 16384u * copied, 16384u,
+                          bars + kBarFull + 8u * copied);
+            }
+            for (uint32_t g = 0; g < 4; ++g) {
+                expect_tx(bars + kBarW1 + 8u * g, 32768u);
+                bulk_load(sb + kOffW1 + 32768u * g, N.wimg + kImgW1 + 32768u * g, 32768u, bars + kBarW1 + 8u * g);
+            }
+            expect_tx(bars + kBarFixed, 8192u);
+            bulk_load(sb + kOffW3, N.wimg + kImgW3, 8192u, bars + kBarFixed);
         }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    for (int i = tid; i < kHid; i += kThreads) {
-        bias[i] = N.b[0][i];
-        bias[kHid + i] = N.b[1][i];
-        bias[2 * kHid + i] = N.b[2][i];
-    }
-    if (tid < kOut) bias[3 * kHid + tid] = N.b[3][tid];
-    if (tid < kIn) {
-        bias[kNormOff + tid] = N.fmean[tid];
-        bias[kNormOff + kIn + tid] = N.fistd[tid];
+        __syncwarp();
+    } else if (warp >= kEpiWarps + 2) {
+        if (both == 1u) {
+            const uint32_t gr = first * (uint32_t)kRows + 32u * (uint32_t)(warp & 3) + (uint32_t)lane;
+#pragma unroll
+            for (int k = 0; k < kIn; ++k) raw_in[k] = gr < P.n ? P.feats[(size_t)gr * kIn + k] : 0.f;
+        }
+    } else {
+        if (warp == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         :: "r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        for (int i = tid; i < kHid; i += (kEpiWarps + 1) * 32) {
+            bias[i] = N.b[0][i];
+            bias[kHid + i] = N.b[1][i];
+            bias[2 * kHid + i] = N.b[2][i];
+        }
+        if (tid < kOut) bias[3 * kHid + tid] = N.b[3][tid];
+        if (tid < kIn) {
+            bias[kNormOff + tid] = N.fmean[tid];
+            bias[kNormOff + kIn + tid] = N.fistd[tid];
+        }
     }
     fence_before();
     __syncthreads();
@@ -343,16 +371,22 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
     if (warp >= kEpiWarps + 2) {
         // ---- in/out warps: warp with quadrant q holds rows 32 q .. +31
         const uint32_t lanes = (32u * (uint32_t)(warp & 3)) << 16, row = 32u * (uint32_t)(warp & 3) + (uint32_t)lane;
-        uint32_t x[2][8];
-        auto load_in = [&](uint32_t t, uint32_t group) {
-            const uint32_t gr = (both * group + t) * (uint32_t)kRows + row;
+        uint32_t x[both][8];
+        auto normalise = [&](uint32_t t, uint32_t group, const float (&v)[kIn]) {
+            const bool in = (both * group + t) * (uint32_t)kRows + row < P.n;
             const float* mean = bias + kNormOff;
             const float* istd = mean + kIn;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                x[t][k] = in ? pack2((v[2 * k] - mean[2 * k]) * istd[2 * k],
+                                     (v[2 * k + 1] - mean[2 * k + 1]) * istd[2 * k + 1]) : 0u;
+        };
+        auto load_in = [&](uint32_t t, uint32_t group) {
+            const uint32_t gr = (both * group + t) * (uint32_t)kRows + row;
             float v[kIn];
 #pragma unroll
-            for (int k = 0; k < kIn; ++k) v[k] = gr < P.n ? (P.feats[(size_t)gr * kIn + k] - mean[k]) * istd[k] : 0.f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) x[t][k] = pack2(v[2 * k], v[2 * k + 1]);
+            for (int k = 0; k < kIn; ++k) v[k] = gr < P.n ? P.feats[(size_t)gr * kIn + k] : 0.f;
+            normalise(t, group, v);
         };
         auto store_in = [&](uint32_t t) {
             tmem_st8(tmem + kColA + 128u * t + lanes, x[t]);
@@ -361,22 +395,22 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
             if (lane == 0) mbar_arrive(bars + kBarIn + 8u * t);
         };
 #pragma unroll
-        for (uint32_t t = 0; t < 2; ++t)
-            if (t < both) {
-                load_in(t, first);
-                store_in(t);
-            }
+        for (uint32_t t = 0; t < both; ++t) {
+            if (both == 1u) normalise(t, first, raw_in);
+            else load_in(t, first);
+            store_in(t);
+        }
         uint32_t k = 0;
 #pragma unroll 1
         for (uint32_t group = first; group < n_groups && ok; group += stride, ++k) {
             const bool more = group + stride < n_groups;
 #pragma unroll
-            for (uint32_t t = 0; t < 2; ++t)
-                if (more && t < both) load_in(t, group + stride);
+            for (uint32_t t = 0; t < both; ++t)
+                if (more) load_in(t, group + stride);
 #pragma unroll
-            for (uint32_t t = 0; t < 2; ++t) {
+            for (uint32_t t = 0; t < both; ++t) {
                 const uint32_t blk = both * group + t;
-                if (t >= both || blk >= n_blocks || !ok) break;
+                if (blk >= n_blocks || !ok) break;
                 ok = mbar_wait(bars + kBarOut + 8u * t, k & 1u, kLimit);
                 if (!ok) break;
                 fence_after();
@@ -398,7 +432,7 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
     } else if (warp == kEpiWarps + 1) {
         // ---- weight copies, in the order the MMA warp uses them
         if (elect_one()) {
-            uint32_t use = 0;
+            uint32_t use = copied;
             auto copy = [&](const unsigned char* src) {
                 const uint32_t s = use % kSlots;
                 if (ok && use >= kSlots) ok = mbar_wait(bars + kBarFree + 8u * s, (use / kSlots - 1u) & 1u, kLimit);
@@ -409,15 +443,9 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
             };
 #pragma unroll 1
             for (uint32_t group = first; group < n_groups && ok; group += stride) {
-                copy(N.wimg + kImgW0);
-                copy(N.wimg + kImgW0 + 16384u);
-                if (group == first) {
-                    for (uint32_t g = 0; g < 4; ++g) {
-                        expect_tx(bars + kBarW1 + 8u * g, 32768u);
-                        bulk_load(sb + kOffW1 + 32768u * g, N.wimg + kImgW1 + 32768u * g, 32768u, bars + kBarW1 + 8u * g);
-                    }
-                    expect_tx(bars + kBarFixed, 8192u);
-                    bulk_load(sb + kOffW3, N.wimg + kImgW3, 8192u, bars + kBarFixed);
+                if (group != first) {
+                    copy(N.wimg + kImgW0);
+                    copy(N.wimg + kImgW0 + 16384u);
                 }
 #pragma unroll 1
                 for (uint32_t i = 0; i < 8; ++i)   // half i / 4, K-block i % 4
@@ -438,7 +466,63 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
             bool fixed = false;
 #pragma unroll 1
             for (uint32_t group = first; group < n_groups && ok; group += stride, ++k) {
-                const uint32_t nt = min(both, n_blocks - both * group);
+                if (both == 1u) {
+                    // One block: its halves have an accumulator each.  The next
+                    // layer's first half starts on the first half of K while the
+                    // epilogue is at the second.
+                    ok = mbar_wait(bars + kBarIn, k & 1u, kLimit);
+#pragma unroll 1
+                    for (uint32_t h = 0; h < 2 && ok; ++h, ++use) {   // K = 16
+                        const uint32_t s = use % kSlots;
+                        ok = mbar_wait(bars + kBarFull + 8u * s, (use / kSlots) & 1u, kLimit);
+                        if (!ok) break;
+                        fence_after();
+                        mma(tmem + kColD + 128u * h, tmem + kColA, ring + 1024u * s, id_half, 0u);
+                        mma_commit(bars + kBarD + 8u * h);
+                        mma_commit(bars + kBarFree + 8u * s);
+                    }
+#pragma unroll 1
+                    for (uint32_t l = 1; l < 3 && ok; ++l) {
+                        if (l == 1 && !fixed)
+                            for (uint32_t g = 0; g < 4 && ok; ++g) ok = mbar_wait(bars + kBarW1 + 8u * g, 0u, kLimit);
+#pragma unroll 1
+                        for (uint32_t q = 0; q < 4 && ok; ++q) {   // half q / 2 over half q % 2 of K
+                            const uint32_t h = q >> 1, g = 2u * (q & 1u);
+                            const uint32_t d = tmem + kColD + 128u * h, a = tmem + kColA + 32u * g;
+                            uint64_t w[2] = {w1 + 2048u * g + 1024u * h, w1 + 2048u * (g + 1u) + 1024u * h};
+                            if (q < 2) ok = mbar_wait(bars + kBarAct + 8u * q, (3u * k + l - 1u) & 1u, kLimit);
+                            if (l == 2)
+#pragma unroll
+                                for (uint32_t e = 0; e < 2; ++e) {
+                                    const uint32_t s = (use + e) % kSlots;
+                                    w[e] = ring + 1024u * s;
+                                    ok = ok && mbar_wait(bars + kBarFull + 8u * s, ((use + e) / kSlots) & 1u, kLimit);
+                                }
+                            if (!ok) break;
+                            fence_after();
+#pragma unroll
+                            for (uint32_t j = 0; j < 8; ++j)
+                                mma(d, a + 8u * j, w[j >> 2] + 2u * (j & 3u), id_half, (g | j) ? 1u : 0u);
+                            if (q & 1u) mma_commit(bars + kBarD + 8u * h);
+                            if (l == 2)
+                                for (uint32_t e = 0; e < 2; ++e, ++use) mma_commit(bars + kBarFree + 8u * (use % kSlots));
+                        }
+                    }
+                    if (ok && !fixed) {
+                        ok = mbar_wait(bars + kBarFixed, 0u, kLimit);
+                        fixed = ok;
+                    }
+                    for (uint32_t h = 0; h < 2 && ok; ++h)
+                        ok = mbar_wait(bars + kBarAct + 8u * h, (3u * k + 2u) & 1u, kLimit);
+                    if (!ok) break;
+                    fence_after();
+#pragma unroll
+                    for (uint32_t i = 0; i < 16; ++i)
+                        mma(tmem + kColD, tmem + kColA + 8u * i, w3 + 128u * (i >> 2) + 2u * (i & 3u), id_out, i ? 1u : 0u);
+                    mma_commit(bars + kBarOut);
+                    continue;
+                }
+                const uint32_t nt = min(2u, n_blocks - 2u * group);
                 // first layer, K = 16
 #pragma unroll 1
                 for (uint32_t h = 0; h < 2 && ok; ++h, ++use) {
@@ -525,8 +609,36 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
         const uint32_t lanes = (32u * (uint32_t)(warp & 3)) << 16;
         const uint32_t d = tmem + kColD + 128u * t + lanes + 64u * sub, a = tmem + kColA + 128u * t + lanes + 32u * sub;
         uint32_t k = 0;
+        if (both == 1u) {
+            // one block: warps 0..7 take its first half, 8..15 its second
+            const uint32_t a1 = tmem + kColA + lanes + 64u * t + 32u * sub;
 #pragma unroll 1
-        for (uint32_t group = first; t < both && both * group + t < n_blocks && ok; group += stride, ++k) {
+            for (uint32_t blk = first; blk < n_blocks && ok; blk += stride, ++k) {
+#pragma unroll 1
+                for (uint32_t l = 0; l < 3; ++l) {
+                    const float* b = bias + l * kHid + 128u * t + 64u * sub;
+                    const uint32_t par = (3u * k + l) & 1u;
+                    uint32_t z[32], w0[16], w1[16];
+                    ok = mbar_wait(bars + kBarD + 8u * t, par, kLimit);
+                    if (!ok) break;
+                    fence_after();
+                    tmem_ld32(d, z);
+                    silu32(z, b, w0);
+                    tmem_ld32(d + 32u, z);
+                    silu32(z, b + 32, w1);
+                    if (t == 0u) ok = mbar_wait(bars + kBarD + 8u, par, kLimit);   // the A operand is free now
+                    if (!ok) break;
+                    fence_after();
+                    tmem_st16(a1, w0);
+                    tmem_st16(a1 + 16u, w1);
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bars + kBarAct + 8u * t);
+                }
+            }
+        }
+#pragma unroll 1
+        for (uint32_t group = first; both == 2u && 2u * group + t < n_blocks && ok; group += stride, ++k) {
 #pragma unroll 1
             for (uint32_t l = 0; l < 3; ++l) {
                 const float* b = bias + l * kHid + 64u * sub;
@@ -599,20 +711,37 @@ cudaError_t launch_pack_sw128(const void* src, int rows, int K, int ld, int kpad
 
 size_t mlp_tc_image_bytes() { return tc::kImgBytes; }
 
-static cudaError_t launch_mlp(MlpParams P, cudaStream_t s)
+// The kernel's shared-memory attribute and the SM count, once per device
+// (first 16): host calls that would otherwise precede every launch.
+static cudaError_t mlp_sms(int* sms)
 {
-    cudaError_t e = cudaFuncSetAttribute(mlp_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)tc::kSmemBytes);
+    constexpr int kDevCache = 16;
+    static std::atomic<int> known[kDevCache];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 1;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if (dev < kDevCache && (*sms = known[dev].load(std::memory_order_acquire)) > 0) return cudaSuccess;
+    e = cudaFuncSetAttribute(mlp_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kSmemBytes);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(mlp_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kSmemBytes);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if (dev < kDevCache) known[dev].store(*sms, std::memory_order_release);
+    return cudaSuccess;
+}
+
+static cudaError_t launch_mlp(const MlpParams& P, cudaStream_t s)
+{
+    int sms = 1;
+    const cudaError_t e = mlp_sms(&sms);
+    if (e != cudaSuccess) return e;
     // one CTA per SM; two blocks in flight where there are more than CTAs
     const uint32_t blocks = (P.n + tc::kRows - 1) / tc::kRows;
     const uint32_t per_net = std::max(1u, (uint32_t)sms / P.n_nets);
-    P.in_flight = blocks > per_net ? 2u : 1u;
-    const uint32_t groups = (blocks + P.in_flight - 1) / P.in_flight;
-    mlp_tc_kernel<<<std::min(groups, per_net) * P.n_nets, tc::kThreads, tc::kSmemBytes, s>>>(P);
+    if (blocks > per_net)
+        mlp_tc_kernel<2><<<std::min((blocks + 1) / 2, per_net) * P.n_nets, tc::kThreads, tc::kSmemBytes, s>>>(P);
+    else
+        mlp_tc_kernel<1><<<blocks * P.n_nets, tc::kThreads, tc::kSmemBytes, s>>>(P);
     return cudaGetLastError();
 }
 
@@ -621,8 +750,21 @@ cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, co
                           float* out, unsigned* err, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    MlpParams P{feats, n, 1u, 1u, {}, err};
+    MlpParams P{feats, n, 1u, {}, err};
     P.net[0] = MlpNet{fmean, fistd, static_cast<const unsigned char*>(wimg), {b0, b1, b2, b3}, out};
+    return launch_mlp(P, s);
+}
+
+cudaError_t launch_mlp_nets(const float* feats, uint32_t n, const PredictNet* nets, int n_nets, unsigned* err,
+                            cudaStream_t s)
+{
+    if (n == 0) return cudaSuccess;
+    MlpParams P{feats, n, (uint32_t)n_nets, {}, err};
+    for (int k = 0; k < n_nets; ++k) {
+        const PredictNet& N = nets[k];
+        P.net[k] = MlpNet{N.fmean, N.fistd, static_cast<const unsigned char*>(N.image), {N.b[0], N.b[1], N.b[2], N.b[3]},
+                          N.z};
+    }
     return launch_mlp(P, s);
 }
 

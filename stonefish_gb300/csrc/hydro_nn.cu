@@ -15,7 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/stonefish_hydro.h"
-#include "hydro_device.cuh"
+#include "hydro_internal.h"
 #include "hydro_mma.cuh"
 
 namespace sfh {
@@ -415,31 +415,13 @@ constexpr int kFeatWords = 18;
 constexpr int kFeatStride = kFeatWords + 1;   // odd: 8-byte reads of a warp free of bank conflicts
 constexpr int kFeatBlock = 128;
 static_assert(offsetof(hydro_body, T_CG) == 0 && offsetof(hydro_body, v) == 33 * 8 &&
-                  offsetof(hydro_body, omega) == 36 * 8 && sizeof(hydro_body) % 8 == 0,
+                  offsetof(hydro_body, omega) == 36 * 8 && offsetof(hydro_body, aabb_min) == 50 * 8 &&
+                  offsetof(hydro_body, aabb_max) == 53 * 8 && sizeof(hydro_body) % 8 == 0,
               "feature words of hydro_body");
 
-__global__ void __launch_bounds__(kFeatBlock) features_kernel(const hydro_body* __restrict__ bodies, uint32_t n,
-                                                              OceanDev o, float* __restrict__ f)
+// The features of a state from its 18 staged words.
+__device__ __forceinline__ void state_features(const double* sw, const OceanDev& o, float (&o16)[16])
 {
-    // Each warp first copies the feature words of its 32 records into shared
-    // memory, consecutive lanes reading consecutive words, so that a load
-    // instruction touches two records instead of 32 (the records may be
-    // page-locked host memory read in place).
-    __shared__ double stage[kFeatBlock / 32][32 * kFeatStride];
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const uint32_t first = blockIdx.x * kFeatBlock + 32u * wib;
-    const double* words = reinterpret_cast<const double*>(bodies);
-    constexpr uint32_t kRecWords = sizeof(hydro_body) / 8;
-#pragma unroll
-    for (uint32_t j = 0; j < (uint32_t)kFeatWords; ++j) {
-        const uint32_t t = lane + 32u * j, r = t / kFeatWords, p = t % kFeatWords;
-        const uint32_t w = p < 12u ? p : 33u + (p - 12u);
-        if (first + r < n) stage[wib][r * kFeatStride + p] = words[(size_t)(first + r) * kRecWords + w];
-    }
-    __syncwarp();
-    const uint32_t i = first + lane;
-    if (i >= n) return;
-    const double* sw = &stage[wib][lane * kFeatStride];
     double R[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) R[k] = sw[k];
@@ -479,7 +461,6 @@ __global__ void __launch_bounds__(kFeatBlock) features_kernel(const hydro_body* 
         out[1] = (Rf[1] * u0 + Rf[4] * u1) + Rf[7] * u2;
         out[2] = (Rf[2] * u0 + Rf[5] * u1) + Rf[8] * u2;
     };
-    float* o16 = f + (size_t)i * 16;
     o16[0] = (float)z + h;                          // depth below the local surface (NED: surface at -h)
     o16[1] = atan2f(Rf[7], Rf[8]);                  // roll
     o16[2] = asinf(fmaxf(-1.f, fminf(1.f, -Rf[6])));  // pitch
@@ -493,11 +474,68 @@ __global__ void __launch_bounds__(kFeatBlock) features_kernel(const hydro_body* 
     o16[15] = k_al;
 }
 
+// A warp copies the feature words (and, with BOX, the AABB) of its 32 records
+// into shared memory, consecutive lanes reading consecutive words, so that a
+// load instruction touches two records instead of 32 (the records may be
+// page-locked host memory read in place).
+template <bool BOX>
+__device__ __forceinline__ void stage_states(const hydro_body* bodies, uint32_t first, uint32_t n, double* stage)
+{
+    constexpr uint32_t kWords = kFeatWords + (BOX ? 6 : 0), kStride = kWords | 1u;
+    const uint32_t lane = threadIdx.x & 31u;
+    const double* words = reinterpret_cast<const double*>(bodies);
+    constexpr uint32_t kRecWords = sizeof(hydro_body) / 8;
+#pragma unroll
+    for (uint32_t j = 0; j < kWords; ++j) {
+        const uint32_t t = lane + 32u * j, r = t / kWords, p = t % kWords;
+        const uint32_t w = p < 12u ? p : p < 18u ? 33u + (p - 12u) : 50u + (p - 18u);
+        if (first + r < n) stage[r * kStride + p] = words[(size_t)(first + r) * kRecWords + w];
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(kFeatBlock) features_kernel(const hydro_body* __restrict__ bodies, uint32_t n,
+                                                              OceanDev o, float* __restrict__ f)
+{
+    __shared__ double stage[kFeatBlock / 32][32 * kFeatStride];
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+    const uint32_t first = blockIdx.x * kFeatBlock + 32u * wib;
+    stage_states<false>(bodies, first, n, stage[wib]);
+    const uint32_t i = first + lane;
+    if (i >= n) return;
+    float o16[16];
+    state_features(&stage[wib][lane * kFeatStride], o, o16);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) f[(size_t)i * 16 + k] = o16[k];
+}
+
 cudaError_t launch_features(const hydro_body* bodies, uint32_t n, OceanDev o, float* f, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
     features_kernel<<<(n + kFeatBlock - 1) / kFeatBlock, kFeatBlock, 0, s>>>(bodies, n, o, f);
     return cudaGetLastError();
+}
+
+// Whether a feature vector lies inside the box and the Mahalanobis radius.
+__device__ __forceinline__ bool gate_admits(const float (&x)[16], const float* Ps, const float* ls, const float* hs,
+                                            const float* ms, float thresh)
+{
+    float d[16];
+    bool in = true;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        in = in && (x[k] >= ls[k]) && (x[k] <= hs[k]);
+        d[k] = x[k] - ms[k];
+    }
+    float q = 0.f;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        float s = 0.f;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) s += Ps[r * 16 + c] * d[c];
+        q += d[r] * s;
+    }
+    return in && q <= thresh;
 }
 
 // Out-of-distribution gate: mask[i] = 1 when feature vector i lies inside
@@ -518,29 +556,17 @@ __global__ void gate_kernel(const float* __restrict__ f, uint32_t n, const float
     __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float d[16];
-    bool in = true;
+    float x[16];
     const float4* f4 = reinterpret_cast<const float4*>(f + (size_t)i * 16);
 #pragma unroll
-    for (int k4 = 0; k4 < 4; ++k4) {
-        const float4 v = f4[k4];
-        const float xs[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int k = 4 * k4 + j;
-            in = in && (xs[j] >= ls[k]) && (xs[j] <= hs[k]);
-            d[k] = xs[j] - ms[k];
-        }
+    for (int k = 0; k < 4; ++k) {
+        const float4 v = f4[k];
+        x[4 * k] = v.x;
+        x[4 * k + 1] = v.y;
+        x[4 * k + 2] = v.z;
+        x[4 * k + 3] = v.w;
     }
-    float q = 0.f;
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        float s = 0.f;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) s += Ps[r * 16 + c] * d[c];
-        q += d[r] * s;
-    }
-    mask[i] = (in && q <= thresh) ? 1 : 0;
+    mask[i] = gate_admits(x, Ps, ls, hs, ms, thresh) ? 1 : 0;
 }
 
 cudaError_t launch_gate(const float* f, uint32_t n, const float* lo, const float* hi, const float* mean,
@@ -548,6 +574,47 @@ cudaError_t launch_gate(const float* f, uint32_t n, const float* lo, const float
 {
     if (n == 0) return cudaSuccess;
     gate_kernel<<<(n + 127) / 128, 128, 0, s>>>(f, n, lo, hi, mean, P, thresh, mask);
+    return cudaGetLastError();
+}
+
+// Features, gate and INSIDE test of a state in one pass over its record: three
+// launches of 16, 7 and 11 us for 65,536 states, of which the last read the
+// records again, 24 us as one (13 us for 16,384).
+constexpr int kStateWords = kFeatWords + 6, kStateStride = kStateWords | 1;
+
+__global__ void __launch_bounds__(kFeatBlock) states_kernel(const hydro_body* __restrict__ bodies, uint32_t n,
+                                                            OceanDev o, GateParams g, float* __restrict__ f,
+                                                            uint8_t* __restrict__ mask)
+{
+    __shared__ double stage[kFeatBlock / 32][32 * kStateStride];
+    __shared__ float Ps[256], ls[16], hs[16], ms[16];
+    for (int k = threadIdx.x; k < 256; k += kFeatBlock) Ps[k] = g.P[k];
+    if (threadIdx.x < 16) {
+        ls[threadIdx.x] = g.lo[threadIdx.x];
+        hs[threadIdx.x] = g.hi[threadIdx.x];
+        ms[threadIdx.x] = g.mean[threadIdx.x];
+    }
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+    const uint32_t first = blockIdx.x * kFeatBlock + 32u * wib;
+    stage_states<true>(bodies, first, n, stage[wib]);
+    __syncthreads();
+    const uint32_t i = first + lane;
+    if (i >= n) return;
+    const double* sw = &stage[wib][lane * kStateStride];
+    float x[16];
+    state_features(sw, o, x);
+    float4* f4 = reinterpret_cast<float4*>(f + (size_t)i * 16);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f4[k] = make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
+    bool in = gate_admits(x, Ps, ls, hs, ms, g.thresh);
+    if (in && g.inside) in = classify(o, sw + kFeatWords, sw + kFeatWords + 3) != HYDRO_INSIDE;
+    mask[i] = in ? 1 : 0;
+}
+
+cudaError_t launch_states(const hydro_body* bodies, uint32_t n, OceanDev o, const GateParams& g, float* feats,
+                          uint8_t* mask, cudaStream_t s)
+{
+    states_kernel<<<(n + kFeatBlock - 1) / kFeatBlock, kFeatBlock, 0, s>>>(bodies, n, o, g, feats, mask);
     return cudaGetLastError();
 }
 
@@ -721,6 +788,73 @@ cudaError_t launch_ensemble(float* za, const float* zb, int ld, uint32_t n, floa
 {
     if (n == 0) return cudaSuccess;
     ensemble_kernel<<<(n + 127) / 128, 128, 0, s>>>(za, zb, ld, n, inv_fs, inv_ts, tau, mask);
+    return cudaGetLastError();
+}
+
+// What follows the networks, in one pass: ensemble_kernel's mean and gate
+// (z1 null: one network), audit_pick_kernel's sample, the admitted states'
+// outputs (merge_kernel's copy) and route_count_kernel's counts.
+__global__ void __launch_bounds__(kCombineBlock)
+combine_kernel(float* __restrict__ z0, const float* __restrict__ z1, uint32_t n, float inv_fs, float inv_ts, float tau,
+               uint32_t audit_stride, uint32_t audit_phase, float* __restrict__ audit_err, uint8_t* __restrict__ mask,
+               uint32_t* __restrict__ counts, float* __restrict__ out)
+{
+    const uint32_t i = blockIdx.x * kCombineBlock + threadIdx.x;
+    bool reject = false;
+    if (i == 0 && audit_stride) {   // the last sample may lie past the last state
+        const uint32_t last = (n - 1) / audit_stride;
+        if ((uint64_t)last * audit_stride + audit_phase >= n) audit_err[last] = -1.f;
+    }
+    if (i < n) {
+        float a[6];
+        float4* pa = reinterpret_cast<float4*>(z0 + (size_t)i * 16);
+        const float4 a0 = pa[0];
+        const float2 a1 = *reinterpret_cast<const float2*>(pa + 1);
+        a[0] = a0.x; a[1] = a0.y; a[2] = a0.z; a[3] = a0.w; a[4] = a1.x; a[5] = a1.y;
+        reject = mask[i] == 0;
+        if (z1) {
+            const float4* pb = reinterpret_cast<const float4*>(z1 + (size_t)i * 16);
+            const float4 b0 = pb[0];
+            const float2 b1 = *reinterpret_cast<const float2*>(pb + 1);
+            const float b[6] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y};
+            float df = 0.f, dt = 0.f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float x = a[k] - b[k], y = a[3 + k] - b[3 + k];
+                df += x * x;
+                dt += y * y;
+            }
+            const float d = fmaxf(sqrtf(df) * inv_fs, sqrtf(dt) * inv_ts);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) a[k] = 0.5f * (a[k] + b[k]);
+            pa[0] = make_float4(a[0], a[1], a[2], a[3]);
+            *reinterpret_cast<float2*>(pa + 1) = make_float2(a[4], a[5]);
+            reject = reject || d > tau;
+        }
+        uint8_t m = reject ? 0 : 1;
+        if (audit_stride && i >= audit_phase && (i - audit_phase) % audit_stride == 0) {
+            if (!reject) m = 2;   // audited: exact as well; its error is written by the finalisation
+            else audit_err[(i - audit_phase) / audit_stride] = -1.f;
+            reject = true;
+        }
+        mask[i] = m;
+        if (!reject) {
+            float2* o2 = reinterpret_cast<float2*>(out + (size_t)i * 6);
+            o2[0] = make_float2(a[0], a[1]);
+            o2[1] = make_float2(a[2], a[3]);
+            o2[2] = make_float2(a[4], a[5]);
+        }
+    }
+    const int c = __syncthreads_count(reject);
+    if (threadIdx.x == 0) counts[blockIdx.x] = (uint32_t)c;
+}
+
+cudaError_t launch_combine(float* z0, const float* z1, uint32_t n, float inv_fs, float inv_ts, float tau,
+                           uint32_t audit_stride, uint32_t audit_phase, float* audit_err, uint8_t* mask,
+                           uint32_t* counts, float* out, cudaStream_t s)
+{
+    combine_kernel<<<(n + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, s>>>(
+        z0, z1, n, inv_fs, inv_ts, tau, audit_stride, audit_phase, audit_err, mask, counts, out);
     return cudaGetLastError();
 }
 

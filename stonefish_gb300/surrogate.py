@@ -551,11 +551,38 @@ class GatedPredictor:
         if self.audit_k:
             self.audit_idx = torch.zeros(self.audit_k, dtype=torch.int32, device=dev)
             self.audit_err = torch.full((audit_ring, self.audit_k), -1.0, dtype=torch.float32, device=dev)
+        if tensor_cores == "tcgen05":
+            self.rows = torch.zeros(n, dtype=torch.int32, device=dev)
+
+    def _predictor(self, split_chunks: bool) -> abi.NnPredictor:
+        """The networks, gates and work buffers as hydro_nn_predict reads them."""
+        p, b = abi.NnPredictor(), self.bufs
+        p.n, p.gate_inside, p.tau, p.audit_stride = self.n, int(self.gate_inside), self.tau, self.audit_stride
+        p.split_chunks = int(split_chunks)
+        p.force_scale, p.torque_scale = self.fs, self.ts
+        g = self.s.gate
+        p.threshold = g["thr"]
+        p.lo, p.hi, p.mean, p.precision = (g[k].data_ptr() for k in ("lo", "hi", "mean", "P"))
+        nets = [(self.s, self.tcw, self.z16)]
+        if self.second is not None:
+            nets.append((self.second, self.tcw2, self.z16b))
+        p.n_nets = len(nets)
+        for d, (net, tcw, z) in zip(p.net, nets):
+            d.fmean, d.fistd, d.image = net.f_mean.data_ptr(), net.f_istd.data_ptr(), tcw["image"].data_ptr()
+            for k in range(4):
+                d.bias[k] = tcw["b"][k].data_ptr()
+            d.z = z.data_ptr()
+        p.err = self.tcw["err"].data_ptr()
+        p.features, p.mask = b["feats"].data_ptr(), b["mask"].data_ptr()
+        for k in ("counts", "packed", "pos", "rows", "n_packed", "out"):
+            setattr(p, k, getattr(self, k).data_ptr())
+        p.exact = self.exact_io.data_ptr()
+        return p
 
     def _ck(self, st):
         _check(self.lib, self.h.ctx, st)
 
-    def predict(self, d_bodies: torch.Tensor) -> torch.Tensor:
+    def predict(self, d_bodies: torch.Tensor, split_chunks: bool = True) -> torch.Tensor:
         """d_bodies: bytes of n hydro_body on the device, or in page-locked
         host memory, which the kernels then read in place (mesh ids are
         ignored: the exact slots use this predictor's mesh).  Returns out
@@ -569,6 +596,16 @@ class GatedPredictor:
             bodies = _ptr(d_bodies)
         else:
             bodies = C.c_void_p(abi.mapped_host_ptr(d_bodies.data_ptr()))
+        if self.mode == "tcgen05":
+            launches = C.c_uint32()
+            row = self.audit_err[self.audit_calls % self.audit_ring] if self.audit_k else None
+            phase = self.audit_calls % self.audit_stride if self.audit_k else 0
+            self._ck(self.lib.hydro_nn_predict(ctx, self.batch.b, C.byref(self._predictor(split_chunks)), bodies,
+                                               C.byref(self.ocean), C.byref(self.settings), phase, _ptr(row),
+                                               C.byref(launches), st))
+            self.audit_calls += 1 if self.audit_k else 0
+            self.launches = launches.value
+            return self.out
         self._ck(self.lib.hydro_nn_features(ctx, bodies, n, C.byref(self.ocean), _ptr(b["feats"]), st))
         self._ck(self.lib.hydro_nn_gate(ctx, _ptr(b["feats"]), n, _ptr(g["lo"]), _ptr(g["hi"]), _ptr(g["mean"]),
                                         _ptr(g["P"]), g["thr"], _ptr(b["mask"]), st))
@@ -576,18 +613,9 @@ class GatedPredictor:
         if self.gate_inside:
             self._ck(self.lib.hydro_nn_gate_inside(ctx, bodies, n, C.byref(self.ocean), _ptr(b["mask"]), st))
             extra += 1
-        if self.mode == "tcgen05":
-            s.infer_tc(b["feats"], self.z16, self.tcw)
-            z, ldz, mlp_launches = self.z16, 16, 1
-            if self.second is not None:
-                self.second.infer_tc(b["feats"], self.z16b, self.tcw2)
-                self._ck(self.lib.hydro_nn_ensemble(ctx, _ptr(self.z16), _ptr(self.z16b), 16, n, self.fs, self.ts,
-                                                    self.tau, _ptr(b["mask"]), st))
-                extra += 2
-        else:
-            s.to_bf16(b["feats"], self.n_pad, N_FEAT, IN_PAD, b["X0"], s.f_mean, s.f_istd)
-            s._mlp(b, self.n_pad)
-            z, ldz, mlp_launches = b["z"], OUT_PAD, 5
+        s.to_bf16(b["feats"], self.n_pad, N_FEAT, IN_PAD, b["X0"], s.f_mean, s.f_istd)
+        s._mlp(b, self.n_pad)
+        z, ldz, mlp_launches = b["z"], OUT_PAD, 5
         if self.audit_k:
             phase = self.audit_calls % self.audit_stride
             self._ck(self.lib.hydro_nn_audit_pick(ctx, _ptr(b["mask"]), n, self.audit_stride, phase, self.audit_k,
@@ -607,7 +635,7 @@ class GatedPredictor:
                                                    st))
             self.audit_calls += 1
             extra += 1
-        # features, gate (+ inside gate, second network, ensemble, audit), network, 2 route, exact step, merge
+        # features, gate (+ inside gate, audit), network, 2 route, exact step, merge
         self.launches = 1 + 1 + mlp_launches + 2 + self.batch.last_launches() + 1 + extra
         return self.out
 

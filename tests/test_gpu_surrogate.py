@@ -656,3 +656,83 @@ def test_audit_pick_and_error(hctx):
         x = max(np.linalg.norm(z[i, :3] - Fb) / fs, np.linalg.norm(z[i, 3:6] - Tb) / ts)
         assert abs(e[j] - x) <= 1e-6 * x + 1e-7
     assert (e > 0).sum() >= picked.size - 1
+
+
+@pytest.mark.parametrize("n,reject,nets,stride", [(1, 0.0, 1, 0), (257, 1.0, 2, 64), (700, 0.02, 2, 64),
+                                                  (6000, 0.002, 1, 1024), (6000, 0.3, 2, 7)])
+def test_fused_prediction_matches_single_entry_points(built_library, n, reject, nets, stride):
+    """hydro_nn_predict against the chain of single entry points it replaces,
+    for one and two networks, with and without the audit, from no state to
+    every state sent to the exact step: same masks, slots, network outputs and
+    audit samples to the bit; the exact rows too, or, where the fused call
+    splits chunks because few states are exact, to the 2e-6 of the force scale
+    that the FP32 summation order is bounded by elsewhere."""
+    from stonefish_gb300.hydro import HydroContext
+    h = HydroContext()
+    mid = h.upload_mesh(*S.hull_mesh(3000))
+    h.set_wave_grid(scenarios.wave_grid(n=256, n_waves=16, seed=5))
+    ocean, st = S.wave_ocean(), scenarios.settings()
+    bodies = S.sample_states(np.random.default_rng(n), n, extent=25.6)
+    bodies["mesh"] = mid
+    d_b = torch.from_numpy(bodies.view(np.uint8).copy()).cuda()
+    P = S._ptr
+    m = max(n, 4096)
+    many = torch.from_numpy(S.sample_states(np.random.default_rng(99), m, extent=25.6).view(np.uint8).copy()).cuda()
+    feats = torch.empty((m, 16), device="cuda")
+    _ck(h, h.lib.hydro_nn_features(h.ctx, P(many), m, C.byref(ocean), P(feats), None))
+    targ = _dev(np.random.default_rng(1).normal(size=(m, 6)) * 500.0)
+    surs = [S.Surrogate(h, batch=256, seed=k) for k in range(nets)]
+    for sur in surs:
+        sur.fit_normalisation(feats, targ, gate_quantile=max(1.0 - reject, 0.0))
+        if reject == 0.0:
+            sur.gate["lo"].fill_(-1e30), sur.gate["hi"].fill_(1e30)
+            sur.gate["thr"] = 1e30
+    second = surs[1] if nets == 2 else None
+    gp = S.GatedPredictor(surs[0], h, mid, n, ocean, st, second=second, tau=1e30 if second else float("inf"),
+                          gate_inside=reject > 0.0, audit_stride=stride)
+    for call in range(2):
+        got = gp.predict(d_b).clone()
+        # the chain
+        f = torch.empty((n, 16), device="cuda")
+        mask = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        g, lib, ctx = surs[0].gate, h.lib, h.ctx
+        _ck(h, lib.hydro_nn_features(ctx, P(d_b), n, C.byref(ocean), P(f), None))
+        _ck(h, lib.hydro_nn_gate(ctx, P(f), n, P(g["lo"]), P(g["hi"]), P(g["mean"]), P(g["P"]), g["thr"], P(mask), None))
+        if gp.gate_inside:
+            _ck(h, lib.hydro_nn_gate_inside(ctx, P(d_b), n, C.byref(ocean), P(mask), None))
+        za = torch.zeros((n, 16), device="cuda")
+        surs[0].infer_tc(f, za, gp.tcw)
+        if second:
+            zb = torch.zeros((n, 16), device="cuda")
+            second.infer_tc(f, zb, gp.tcw2)
+            _ck(h, lib.hydro_nn_ensemble(ctx, P(za), P(zb), 16, n, gp.fs, gp.ts, gp.tau, P(mask), None))
+        idx = torch.zeros(max(gp.audit_k, 1), dtype=torch.int32, device="cuda")
+        if stride:
+            _ck(h, lib.hydro_nn_audit_pick(ctx, P(mask), n, stride, call % stride, gp.audit_k, P(idx), None))
+        cnt = torch.zeros((n + 255) // 256, dtype=torch.int32, device="cuda")
+        packed, pos = torch.zeros_like(d_b), torch.zeros(n, dtype=torch.int32, device="cuda")
+        npk, io = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(n * 168, dtype=torch.uint8, device="cuda")
+        _ck(h, lib.hydro_nn_route(ctx, P(d_b), P(mask), n, P(cnt), P(packed), P(pos), P(npk), P(io), None))
+        gp.batch.compute_device_prefix(packed.data_ptr(), npk.data_ptr(), ocean, st, io.data_ptr())
+        out = torch.zeros((n, 6), device="cuda")
+        _ck(h, lib.hydro_nn_merge(ctx, P(d_b), P(za), 16, P(pos), P(io), n, P(out), None))
+        torch.cuda.synchronize()
+        k = int(npk.item())
+        assert gp.rejected() == k and (reject > 0.0 or k == 0) and (reject < 1.0 or k == n)
+        assert torch.equal(gp.pos, pos) and torch.equal(gp.bufs["mask"][:n], mask)
+        assert torch.equal(gp.bufs["feats"][:n], f) and torch.equal(gp.z16[:n, :6], za[:, :6])
+        adm = pos < 0
+        assert torch.equal(got[adm], out[adm])
+        if k:
+            scale = torch.tensor([gp.fs] * 3 + [gp.ts] * 3, device="cuda")
+            assert float(((got - out)[~adm].abs() / scale).max()) <= 2e-6
+        if stride:
+            err = torch.zeros(gp.audit_k, device="cuda")
+            _ck(h, lib.hydro_nn_audit_error(ctx, P(d_b), P(za), 16, P(pos), P(io), P(idx), gp.audit_k, gp.fs, gp.ts,
+                                            P(err), None))
+            torch.cuda.synchronize()
+            mine = gp.audit_err[call]
+            assert torch.equal(mine < 0, err < 0)
+            assert torch.allclose(mine, err, rtol=0, atol=4e-6)
+    gp.close()
+    h.close()
