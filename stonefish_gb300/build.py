@@ -21,7 +21,7 @@ LIB = os.path.join(LIB_DIR, "libstonefish_hydro.so")
 
 SOURCES = ["hydro_kernels.cu", "hydro_api.cu", "hydro_nn.cu", "hydro_train.cu", "hydro_rollout.cu", "hydro_mlp_tc.cu", "hydro_cable.cu", "hydro_fft_ocean.cu",
            "hydro_ingest.cu", "hydro_approx.cu"]
-HEADERS = ["hydro_device.cuh", "hydro_internal.h", "hydro_pair.cuh", "hydro_mma.cuh", "hydro_train.h"]
+HEADERS = ["hydro_device.cuh", "hydro_internal.h", "hydro_pair.cuh", "hydro_mma.cuh", "hydro_chain.cuh", "hydro_train.h"]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",

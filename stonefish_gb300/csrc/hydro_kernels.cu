@@ -28,6 +28,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "hydro_chain.cuh"
 #include "hydro_internal.h"
 #include "hydro_pair.cuh"
 
@@ -654,6 +655,7 @@ __device__ __forceinline__ void list_chunks(const KParams& P, uint32_t body, con
 // *n_active of them when a device count is given).
 __global__ void prep_kernel(const KParams P)
 {
+    launch_dependents();
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) *P.err = 0u;
         if (threadIdx.x < (unsigned)kClaimClasses) P.work[threadIdx.x] = 0u;
@@ -1174,6 +1176,7 @@ __global__ void __launch_bounds__(kThreads) __maxnreg__(MINB == 2 ? 128 : 255) c
         }
         mbar_fence_init();
     }
+    dependency_wait();
     __syncthreads();
     if (tid >= kBlock) {
         producer(P, S);
@@ -1226,6 +1229,7 @@ __global__ void __launch_bounds__(kBodyThreads) finalize_kernel(const KParams P)
     __shared__ double sums[kPerCta][kPartialStride];
     const int sub = (int)(threadIdx.x % kFinSub), slot = (int)(threadIdx.x / kFinSub);
     const int lane = (int)(threadIdx.x & 31u);
+    dependency_wait();
     if (blockIdx.x == 0 && threadIdx.x < (unsigned)kClaimClasses)
         P.n_listed[threadIdx.x] = 0u;   // the chunk kernel has finished with them
     const uint32_t limit = P.n_active ? min(P.n_bodies, *P.n_active) : P.n_bodies;
@@ -1315,6 +1319,8 @@ predict_pack_kernel(const KParams P, const hydro_body* __restrict__ states, uint
     __shared__ uint32_t sums[2];
     __shared__ uint32_t list[kCombineBlock];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    launch_dependents();
+    dependency_wait();
     if (warp == 0) {   // rejects before this block, and in all
         uint32_t before = 0, total = 0;
         for (uint32_t k = lane; k < n_blocks; k += 32) {
@@ -1453,7 +1459,13 @@ int chunk_kernel_occupancy(int cut64, int waves, int ctas_per_sm, int aero, int 
 // beyond (a device count may leave most of a large batch idle).
 static uint32_t body_cap(LaunchShape shape) { return 8u * (uint32_t)std::max(1, shape.grid / std::max(1, shape.ctas_per_sm)); }
 
-// The chunk kernel and the finalisation of prepared bodies.
+// The chunk kernel and the finalisation of prepared bodies, chained to the
+// preparation: the chunk kernel's CTAs set up their barriers while it runs (a
+// single body's call 43.3 -> 38.8 us, a hull among waves 67.7 -> 60.7, 1,000
+// spheres 46.8 -> 44.4).  The chunk kernel does not trigger early: the
+// finalisation's CTAs would all be placed on the SMs that run out of chunks
+// first (12,288 mixed bodies 268 us, without 259).  With events between the
+// kernels they are launched as usual.
 static cudaError_t launch_chunks(const KParams& P, LaunchShape shape, int cut64, cudaStream_t s, cudaEvent_t* ev)
 {
     cudaError_t e;
@@ -1466,11 +1478,12 @@ static cudaError_t launch_chunks(const KParams& P, LaunchShape shape, int cut64,
     const void* k = chunk_kernel_for(cut64, P.ocean.waves != 0, shape.ctas_per_sm, aero, field);
     if ((e = chunk_kernel_attr(cut64, P.ocean.waves != 0, shape.ctas_per_sm, aero, field))) return e;
     void* args[] = {const_cast<KParams*>(&P)};
-    if ((e = cudaLaunchKernel(k, dim3(grid), dim3(kThreads), args, sizeof(ChunkSmem), s))) return e;
+    if ((e = launch_chained(k, grid, kThreads, sizeof(ChunkSmem), s, args, !ev))) return e;
     if (ev && (e = cudaEventRecord(ev[2], s))) return e;
-    finalize_kernel<<<std::min((P.n_bodies + kBodyThreads / kFinSub - 1) / (kBodyThreads / kFinSub), cap),
-                      kBodyThreads, 0, s>>>(P);
-    if ((e = cudaGetLastError())) return e;
+    if ((e = launch_chained((const void*)finalize_kernel,
+                            std::min((P.n_bodies + kBodyThreads / kFinSub - 1) / (kBodyThreads / kFinSub), cap),
+                            kBodyThreads, 0, s, args, !ev)))
+        return e;
     if (ev && (e = cudaEventRecord(ev[3], s))) return e;
     return cudaSuccess;
 }
@@ -1496,8 +1509,9 @@ cudaError_t launch_predict_step(const KParams& P, const hydro_body* states, uint
                                 uint32_t* n_packed, LaunchShape shape, int cut64, cudaStream_t s)
 {
     const uint32_t nb = (n + kCombineBlock - 1) / kCombineBlock;
-    predict_pack_kernel<<<nb, kCombineBlock, 0, s>>>(P, states, mask, n, counts, nb, packed, pos, rows, n_packed);
-    cudaError_t e = cudaGetLastError();
+    void* args[] = {const_cast<KParams*>(&P), &states, &mask, &n, &counts, const_cast<uint32_t*>(&nb), &packed, &pos,
+                    &rows, &n_packed};
+    const cudaError_t e = launch_chained((const void*)predict_pack_kernel, nb, kCombineBlock, 0, s, args);
     if (e != cudaSuccess) return e;
     return launch_chunks(P, shape, cut64, s, nullptr);
 }

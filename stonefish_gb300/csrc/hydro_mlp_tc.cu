@@ -46,6 +46,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "hydro_chain.cuh"
 #include "hydro_internal.h"
 
 namespace sfh {
@@ -340,6 +341,7 @@ __global__ void __launch_bounds__(tc::kThreads, 1) mlp_tc_kernel(const __grid_co
         }
         __syncwarp();
     } else if (warp >= kEpiWarps + 2) {
+        dependency_wait();   // the only warps that touch what an earlier kernel of the call writes
         if (both == 1u) {
             const uint32_t gr = first * (uint32_t)kRows + 32u * (uint32_t)(warp & 3) + (uint32_t)lane;
 #pragma unroll
@@ -730,7 +732,11 @@ static cudaError_t mlp_sms(int* sms)
     return cudaSuccess;
 }
 
-static cudaError_t launch_mlp(const MlpParams& P, cudaStream_t s)
+// chained: behind the kernel that writes the features, in the same call.  The
+// kernel itself does not trigger early: its CTAs fill their SMs, so that what
+// follows would be placed on the few that have none (16,384 states, 128 CTAs:
+// a rollout step 83 -> 88 us).
+static cudaError_t launch_mlp(const MlpParams& P, cudaStream_t s, bool chained)
 {
     int sms = 1;
     const cudaError_t e = mlp_sms(&sms);
@@ -738,11 +744,12 @@ static cudaError_t launch_mlp(const MlpParams& P, cudaStream_t s)
     // one CTA per SM; two blocks in flight where there are more than CTAs
     const uint32_t blocks = (P.n + tc::kRows - 1) / tc::kRows;
     const uint32_t per_net = std::max(1u, (uint32_t)sms / P.n_nets);
+    void* args[] = {const_cast<MlpParams*>(&P)};
     if (blocks > per_net)
-        mlp_tc_kernel<2><<<std::min((blocks + 1) / 2, per_net) * P.n_nets, tc::kThreads, tc::kSmemBytes, s>>>(P);
-    else
-        mlp_tc_kernel<1><<<blocks * P.n_nets, tc::kThreads, tc::kSmemBytes, s>>>(P);
-    return cudaGetLastError();
+        return launch_chained((const void*)mlp_tc_kernel<2>, std::min((blocks + 1) / 2, per_net) * P.n_nets,
+                              tc::kThreads, tc::kSmemBytes, s, args, chained);
+    return launch_chained((const void*)mlp_tc_kernel<1>, blocks * P.n_nets, tc::kThreads, tc::kSmemBytes, s, args,
+                          chained);
 }
 
 cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, const float* fistd,
@@ -752,7 +759,7 @@ cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, co
     if (n == 0) return cudaSuccess;
     MlpParams P{feats, n, 1u, {}, err};
     P.net[0] = MlpNet{fmean, fistd, static_cast<const unsigned char*>(wimg), {b0, b1, b2, b3}, out};
-    return launch_mlp(P, s);
+    return launch_mlp(P, s, false);
 }
 
 cudaError_t launch_mlp_nets(const float* feats, uint32_t n, const PredictNet* nets, int n_nets, unsigned* err,
@@ -765,7 +772,7 @@ cudaError_t launch_mlp_nets(const float* feats, uint32_t n, const PredictNet* ne
         P.net[k] = MlpNet{N.fmean, N.fistd, static_cast<const unsigned char*>(N.image), {N.b[0], N.b[1], N.b[2], N.b[3]},
                           N.z};
     }
-    return launch_mlp(P, s);
+    return launch_mlp(P, s, true);
 }
 
 }  // namespace sfh

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/stonefish_hydro.h"
+#include "hydro_chain.cuh"
 #include "hydro_internal.h"
 #include "hydro_mma.cuh"
 
@@ -588,6 +589,7 @@ __global__ void __launch_bounds__(kFeatBlock) states_kernel(const hydro_body* __
 {
     __shared__ double stage[kFeatBlock / 32][32 * kStateStride];
     __shared__ float Ps[256], ls[16], hs[16], ms[16];
+    launch_dependents();
     for (int k = threadIdx.x; k < 256; k += kFeatBlock) Ps[k] = g.P[k];
     if (threadIdx.x < 16) {
         ls[threadIdx.x] = g.lo[threadIdx.x];
@@ -801,6 +803,8 @@ combine_kernel(float* __restrict__ z0, const float* __restrict__ z1, uint32_t n,
 {
     const uint32_t i = blockIdx.x * kCombineBlock + threadIdx.x;
     bool reject = false;
+    launch_dependents();
+    dependency_wait();
     if (i == 0 && audit_stride) {   // the last sample may lie past the last state
         const uint32_t last = (n - 1) / audit_stride;
         if ((uint64_t)last * audit_stride + audit_phase >= n) audit_err[last] = -1.f;
@@ -853,9 +857,8 @@ cudaError_t launch_combine(float* z0, const float* z1, uint32_t n, float inv_fs,
                            uint32_t audit_stride, uint32_t audit_phase, float* audit_err, uint8_t* mask,
                            uint32_t* counts, float* out, cudaStream_t s)
 {
-    combine_kernel<<<(n + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, s>>>(
-        z0, z1, n, inv_fs, inv_ts, tau, audit_stride, audit_phase, audit_err, mask, counts, out);
-    return cudaGetLastError();
+    void* args[] = {&z0, &z1, &n, &inv_fs, &inv_ts, &tau, &audit_stride, &audit_phase, &audit_err, &mask, &counts, &out};
+    return launch_chained((const void*)combine_kernel, (n + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, s, args);
 }
 
 // Audit sample: rows phase, phase + stride, ... that the gate admitted are

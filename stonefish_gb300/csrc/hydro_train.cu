@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/stonefish_hydro.h"
+#include "hydro_chain.cuh"
 #include "hydro_mma.cuh"
 #include "hydro_train.h"
 
@@ -53,12 +54,6 @@ __device__ __forceinline__ void cp16(void* dst, const void* src)
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
-
-// Programmatic dependent launch: the step's kernels are a chain, and each is
-// launched while the one before it runs, so that its CTAs are there when the
-// last one of that ends.  Nothing is read or written before dependency_wait().
-__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Chunk i of the weights in the order the row kernel multiplies by them:
 // 64 rows of the layers' weights going forward, of their transposes going
@@ -532,25 +527,15 @@ cudaError_t launch_train_step(const RowsParams& R, const GradsParams& G, const U
     int grads = 256, updates = 4;   // loss blocks; bias blocks
     for (const GradLayer& L : G.layer) grads += (L.k / 64) * (L.n / 64) * L.splits + (L.n / 32) * L.slabs;
     for (const UpdateLayer& L : U.layer) updates += (L.k / 32) * (L.n / 8);
-    cudaLaunchAttribute chain{};
-    chain.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    chain.val.programmaticStreamSerializationAllowed = 1;
-    auto config = [&](int grid, int block, size_t smem) {
-        cudaLaunchConfig_t c{};
-        c.gridDim = dim3(grid);
-        c.blockDim = dim3(block);
-        c.dynamicSmemBytes = smem;
-        c.stream = s;
-        c.attrs = &chain;
-        c.numAttrs = 1;
-        return c;
-    };
-    cudaLaunchConfig_t c = config(R.batch / train::kRows, train::kThreads, train::kRowsSmem);
-    if ((e = cudaLaunchKernelEx(&c, train_rows_kernel, R)) != cudaSuccess) return e;
-    c = config(grads, train::kGradThreads, 0);
-    if ((e = cudaLaunchKernelEx(&c, train_grads_kernel, G)) != cudaSuccess) return e;
-    c = config(updates, 256, 0);
-    return cudaLaunchKernelEx(&c, train_update_kernel, U);
+    // chained from step to step: the first kernel too reads nothing before its wait
+    void* ar[] = {const_cast<RowsParams*>(&R)};
+    void* ag[] = {const_cast<GradsParams*>(&G)};
+    void* au[] = {const_cast<UpdateParams*>(&U)};
+    if ((e = launch_chained((const void*)train_rows_kernel, R.batch / train::kRows, train::kThreads, train::kRowsSmem, s,
+                            ar)))
+        return e;
+    if ((e = launch_chained((const void*)train_grads_kernel, grads, train::kGradThreads, 0, s, ag))) return e;
+    return launch_chained((const void*)train_update_kernel, updates, 256, 0, s, au);
 }
 
 }  // namespace sfh
