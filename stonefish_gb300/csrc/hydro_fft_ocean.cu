@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 #include <vector>
 
+#include "hydro_chain.cuh"
 #include "hydro_internal.h"
 
 namespace sfh {
@@ -164,12 +165,10 @@ void fft_ocean_butterfly(int passes, std::vector<int2>& idx, std::vector<float2>
     }
 }
 
-// oceanInit.frag: h(k,t) of the four grids, (h1 + i h2, h3 + i h4)
-__global__ void fft_init_kernel(const float4* __restrict__ s12, const float4* __restrict__ s34, int N, float4 inv_grid,
-                                float t, float4* __restrict__ out)
+// oceanInit.frag: h(k,t) of the four grids at texel (x, y), (h1 + i h2, h3 + i h4)
+__device__ __forceinline__ float4 fft_init(const float4* __restrict__ s12, const float4* __restrict__ s34, int N,
+                                           const float4& inv_grid, float t, int x, int y)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= N) return;
     const float Nf = (float)N;
     const float tx = (x + 0.5f) / Nf, ty = (y + 0.5f) / Nf;
     const float stx = floorf(tx * Nf) / Nf, sty = floorf(ty * Nf) / Nf;
@@ -182,61 +181,87 @@ __global__ void fft_init_kernel(const float4* __restrict__ s12, const float4* __
     const float sc[4][2] = {{ac.x * r2, ac.y * r2}, {ac.z * r2, ac.w * r2}, {bc.x * r2, bc.y * r2}, {bc.z * r2, bc.w * r2}};
     const float ig[4] = {inv_grid.x, inv_grid.y, inv_grid.z, inv_grid.w};
     float h[4][2];
+#pragma unroll
     for (int g = 0; g < 4; ++g) {
         const float kx = X * ig[g], ky = Y * ig[g];
         const float K = sqrtf(kx * kx + ky * ky);
         const float w = sqrtf(9.81f * K * (1.0f + K * K / (370.0f * 370.0f)));
-        const float c = cosf(w * t), s = sinf(w * t);
+        float s, c;
+        sincosf(w * t, &s, &c);
         h[g][0] = (s0[g][0] + sc[g][0]) * c - (s0[g][1] + sc[g][1]) * s;
         h[g][1] = (s0[g][0] - sc[g][0]) * s + (s0[g][1] - sc[g][1]) * c;
     }
-    out[(size_t)y * N + x] = make_float4(h[0][0] + -h[1][1], h[0][1] + h[1][0], h[2][0] + -h[3][1], h[2][1] + h[3][0]);
+    return make_float4(h[0][0] + -h[1][1], h[0][1] + h[1][0], h[2][0] + -h[3][1], h[2][1] + h[3][0]);
 }
 
-// oceanFFTX.frag / oceanFFTY.frag: all passes of one line in shared memory
-__global__ void fft_lines_kernel(float4* __restrict__ data, int N, int passes, const int2* __restrict__ idx,
-                                 const float2* __restrict__ w, int vertical)
+// oceanFFTX.frag / oceanFFTY.frag: all passes of a CTA's lines in shared
+// memory.  The rows (VERTICAL false) are formed in place from the spectrum
+// instead of by a launch of their own, and a CTA takes two columns, whose
+// 16-byte texels share 32-byte sectors.  A pass's butterfly entries are loaded
+// before the barrier that ends the pass before it, so that no pass waits for
+// L2.  256 x 256 texels: init, rows and columns 5.5 + 7.7 + 8.2 us, now 8.0 +
+// 7.3 us, and the columns' launch is chained to the rows.
+template <bool VERTICAL>
+__global__ void fft_lines_kernel(const float4* __restrict__ s12, const float4* __restrict__ s34, float4 inv_grid,
+                                 float t, float4* __restrict__ data, int N, int passes, const int2* __restrict__ idx,
+                                 const float2* __restrict__ w)
 {
     extern __shared__ float4 line[];
+    constexpr int kLines = VERTICAL ? 2 : 1;
+    const int n = kLines * N;                        // texel e of the CTA: line e % kLines, position e / kLines
     float4* a = line;
-    float4* b = line + N;
-    const int l = blockIdx.x;
-    for (int p = threadIdx.x; p < N; p += blockDim.x)
-        a[p] = data[vertical ? (size_t)p * N + l : (size_t)l * N + p];
+    float4* b = line + n;
+    const int l = blockIdx.x * kLines;
+    const bool one = n <= (int)blockDim.x;           // one texel per thread
+    int2 j = make_int2(0, 0);
+    float2 ww = make_float2(0.f, 0.f);
+    auto entry = [&](int pass, int e) {
+        j = idx[(size_t)pass * N + e / kLines];
+        ww = w[(size_t)pass * N + e / kLines];
+    };
+    if (one && (int)threadIdx.x < n) entry(0, threadIdx.x);
+    if (VERTICAL) dependency_wait();
+    else launch_dependents();
+    for (int e = threadIdx.x; e < n; e += blockDim.x)
+        a[e] = VERTICAL ? data[(size_t)(e / kLines) * N + l + e % kLines] : fft_init(s12, s34, N, inv_grid, t, e, l);
     __syncthreads();
     for (int pass = 0; pass < passes; ++pass) {
-        for (int p = threadIdx.x; p < N; p += blockDim.x) {
-            const int2 j = idx[(size_t)pass * N + p];
-            const float2 ww = w[(size_t)pass * N + p];
-            const float4 i1 = a[j.x], i2 = a[j.y];
+        for (int e = threadIdx.x; e < n; e += blockDim.x) {
+            if (!one) entry(pass, e);
+            const float4 i1 = a[j.x * kLines + e % kLines], i2 = a[j.y * kLines + e % kLines];
             const float r1x = ww.x * i2.x - ww.y * i2.y;
             const float r1y = ww.y * i2.x + ww.x * i2.y;
             const float r2x = ww.x * i2.z - ww.y * i2.w;
             const float r2y = ww.y * i2.z + ww.x * i2.w;
-            b[p] = make_float4(i1.x + r1x, i1.y + r1y, i1.z + r2x, i1.w + r2y);
+            b[e] = make_float4(i1.x + r1x, i1.y + r1y, i1.z + r2x, i1.w + r2y);
+            if (one && pass + 1 < passes) entry(pass + 1, e);
         }
         __syncthreads();
-        float4* t = a;
+        float4* swap = a;
         a = b;
-        b = t;
+        b = swap;
     }
-    for (int p = threadIdx.x; p < N; p += blockDim.x)
-        data[vertical ? (size_t)p * N + l : (size_t)l * N + p] = a[p];
+    for (int e = threadIdx.x; e < n; e += blockDim.x)
+        data[VERTICAL ? (size_t)(e / kLines) * N + l + e % kLines : (size_t)l * N + e] = a[e];
 }
 
 cudaError_t launch_fft_ocean(const float4* s12, const float4* s34, const int2* idx, const float2* w, int passes,
                              float4 inv_grid, float t, float4* out, cudaStream_t s)
 {
-    const int N = 1 << passes;
-    const int tpb = N < 256 ? N : 256;
-    fft_init_kernel<<<dim3((N + tpb - 1) / tpb, N), tpb, 0, s>>>(s12, s34, N, inv_grid, t, out);
-    cudaError_t e = cudaGetLastError();
+    const int N = 1 << passes;   // at least 2, so the columns pair up
+    const size_t line = 2 * (size_t)N * sizeof(float4);
+    const int tx = N < 512 ? N : 512, ty = 2 * N < 512 ? 2 * N : 512;
+    cudaError_t e = cudaSuccess;
+    if (2 * line > 48 * 1024)
+        e = cudaFuncSetAttribute(fft_lines_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * line));
+    if (e == cudaSuccess && line > 48 * 1024)
+        e = cudaFuncSetAttribute(fft_lines_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)line);
     if (e != cudaSuccess) return e;
-    const size_t smem = 2 * (size_t)N * sizeof(float4);
-    fft_lines_kernel<<<N, tpb, smem, s>>>(out, N, passes, idx, w, 0);
+    fft_lines_kernel<false><<<N, tx, line, s>>>(s12, s34, inv_grid, t, out, N, passes, idx, w);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    fft_lines_kernel<<<N, tpb, smem, s>>>(out, N, passes, idx, w, 1);
-    return cudaGetLastError();
+    int n = N;
+    void* args[] = {&s12, &s34, &inv_grid, &t, &out, &n, &passes, &idx, &w};
+    return launch_chained((const void*)fft_lines_kernel<true>, N / 2, ty, 2 * line, s, args);
 }
 
 }  // namespace sfh
