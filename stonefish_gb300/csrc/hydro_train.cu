@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
 namespace train {
 
 constexpr int kGradThreads = 128;
-constexpr int kGradStages = 4;
+constexpr int kGradStages = 3;
 constexpr int kGradLd = 64 + 8;
 
 struct GradSmem {
@@ -405,7 +405,7 @@ __device__ __forceinline__ void loss_block(float* red, const GradsParams& P, int
 
 }  // namespace train
 
-__global__ void __launch_bounds__(train::kGradThreads) train_grads_kernel(const GradsParams P)
+__global__ void __launch_bounds__(train::kGradThreads, 7) train_grads_kernel(const GradsParams P)
 {
     using namespace train;
     __shared__ __align__(16) union {
@@ -417,6 +417,17 @@ __global__ void __launch_bounds__(train::kGradThreads) train_grads_kernel(const 
     launch_dependents();
     // the short CTAs first, so that they run beside the products
     int b = (int)blockIdx.x;
+#pragma unroll 1
+    for (int l = 0; l < 4; ++l) {
+        const GradLayer& L = P.layer[l];
+        const int tn = L.n / 64, tiles = (L.k / 64) * tn, count = tiles * L.splits;
+        if (b < count) {
+            const int t = b % tiles;
+            weight_tile(S.g, L, (t / tn) * 64, (t % tn) * 64, b / tiles);
+            return;
+        }
+        b -= count;
+    }
     if (b < 256) {
         loss_block(S.red, P, b);
         return;
@@ -428,17 +439,6 @@ __global__ void __launch_bounds__(train::kGradThreads) train_grads_kernel(const 
         const int groups = L.n / 32, count = groups * L.slabs;
         if (b < count) {
             column_slab(S.part, L, (b % groups) * 32, b / groups, P.batch);
-            return;
-        }
-        b -= count;
-    }
-#pragma unroll 1
-    for (int l = 0; l < 4; ++l) {
-        const GradLayer& L = P.layer[l];
-        const int tn = L.n / 64, tiles = (L.k / 64) * tn, count = tiles * L.splits;
-        if (b < count) {
-            const int t = b % tiles;
-            weight_tile(S.g, L, (t / tn) * 64, (t % tn) * 64, b / tiles);
             return;
         }
         b -= count;
@@ -483,11 +483,10 @@ __device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int 
 
 // A CTA updates 32 x 8 weights (the transposed copy leaves through shared
 // memory in 64-byte rows) or, the last four CTAs, one layer's biases.
-__global__ void __launch_bounds__(256) train_update_kernel(const UpdateParams P)
+__global__ void __launch_bounds__(256, 5) train_update_kernel(const UpdateParams P)
 {
     using namespace train;
     __shared__ bf16 tile[8][34];
-    dependency_wait();
     launch_dependents();
     int b = (int)blockIdx.x;
     const int tid = threadIdx.x;
@@ -499,6 +498,7 @@ __global__ void __launch_bounds__(256) train_update_kernel(const UpdateParams P)
             const int r = (b / tn) * 32 + (tid >> 3), c = (b % tn) * 8 + (tid & 7);
             const size_t i = (size_t)r * L.n + c, mn = (size_t)L.k * L.n;
             const Moments o{L.w[i], L.mw[i], L.vw[i]};
+            dependency_wait();
             const float g = ordered_sum(L.part + i, mn, L.splits);
             L.gw[i] = g;
             const bf16 h = __float2bfloat16(adamw(P, o, L.w, L.mw, L.vw, i, g, P.wd));
@@ -510,6 +510,7 @@ __global__ void __launch_bounds__(256) train_update_kernel(const UpdateParams P)
         }
         b -= count;
     }
+    dependency_wait();
     const UpdateLayer& L = P.layer[b];
     for (int c = tid; c < L.n; c += 256) {
         const Moments o{L.b[c], L.mb[c], L.vb[c]};
