@@ -5,7 +5,7 @@
 // Step by step the layers' products, epilogues, transposes, column sums and
 // parameter updates are 36 launches of 3 to 15 us whose operands travel
 // through memory between them: 228 us at batch 4096, of which the tensor
-// cores need about 3; the fused step takes 47 us.  Here
+// cores need about 3; the fused step takes 42 us.  Here
 //   1. train_rows_kernel: 32 rows of the batch go through the four layers,
 //      the loss gradient and back to the first layer's pre-activations in
 //      one CTA.  No row needs another one, so the activations stay in shared
@@ -269,6 +269,8 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
 namespace train {
 
 constexpr int kGradThreads = 128;
+// Three stages and 72 registers let seven CTAs run per SM: with four stages,
+// and so six CTAs, a step took 1 us longer; eight CTAs spill.
 constexpr int kGradStages = 3;
 constexpr int kGradLd = 64 + 8;
 
@@ -415,7 +417,7 @@ __global__ void __launch_bounds__(train::kGradThreads, 7) train_grads_kernel(con
     } S;
     dependency_wait();
     launch_dependents();
-    // the short CTAs first, so that they run beside the products
+    // the products first: behind the short CTAs their last wave is emptier (a step 1 us longer)
     int b = (int)blockIdx.x;
 #pragma unroll 1
     for (int l = 0; l < 4; ++l) {
@@ -482,7 +484,12 @@ __device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int 
 }  // namespace train
 
 // A CTA updates 32 x 8 weights (the transposed copy leaves through shared
-// memory in 64-byte rows) or, the last four CTAs, one layer's biases.
+// memory in 64-byte rows) or, the last four CTAs, one layer's biases.  Five
+// CTAs per SM take the 644 in one wave; with the four that unbounded registers
+// allow a second wave held 36 of them (10.8 us, now 7.8).  The parameters are
+// read before the wait: the step's row kernel has waited for the update that
+// wrote them, and this kernel is placed when the gradients' have all waited
+// for the row kernel.
 __global__ void __launch_bounds__(256, 5) train_update_kernel(const UpdateParams P)
 {
     using namespace train;
