@@ -442,11 +442,10 @@ __device__ __forceinline__ void state_features(const double* sw, const OceanDev&
     if (o.waves) {
         const float a = kWaveReach;
         const float fx = (float)x, fy = (float)y;
+        const float2 al = wave_height2(o, make_float2(fx + a * ux, fx - a * ux), make_float2(fy + a * uy, fy - a * uy));
+        const float2 ac = wave_height2(o, make_float2(fx - a * uy, fx + a * uy), make_float2(fy + a * ux, fy - a * ux));
         h = -wave_height(o, fx, fy);
-        const float ef = -wave_height(o, fx + a * ux, fy + a * uy);
-        const float eb = -wave_height(o, fx - a * ux, fy - a * uy);
-        const float el = -wave_height(o, fx - a * uy, fy + a * ux);
-        const float er = -wave_height(o, fx + a * uy, fy - a * ux);
+        const float ef = -al.x, eb = -al.y, el = -ac.x, er = -ac.y;
         s_al = (ef - eb) / (2.f * a);
         s_ac = (el - er) / (2.f * a);
         k_al = (ef + eb - 2.f * h) / (a * a);
@@ -475,22 +474,21 @@ __device__ __forceinline__ void state_features(const double* sw, const OceanDev&
     o16[15] = k_al;
 }
 
-// A warp copies the feature words (and, with BOX, the AABB) of its 32 records
-// into shared memory, consecutive lanes reading consecutive words, so that a
+// A warp copies the words FIRST .. FIRST + COUNT - 1 of its 32 records (the
+// feature words, then the AABB) into shared memory, consecutive lanes reading consecutive words, so that a
 // load instruction touches two records instead of 32 (the records may be
 // page-locked host memory read in place).
-template <bool BOX>
+template <uint32_t FIRST, uint32_t COUNT, uint32_t STRIDE>
 __device__ __forceinline__ void stage_states(const hydro_body* bodies, uint32_t first, uint32_t n, double* stage)
 {
-    constexpr uint32_t kWords = kFeatWords + (BOX ? 6 : 0), kStride = kWords | 1u;
     const uint32_t lane = threadIdx.x & 31u;
     const double* words = reinterpret_cast<const double*>(bodies);
     constexpr uint32_t kRecWords = sizeof(hydro_body) / 8;
 #pragma unroll
-    for (uint32_t j = 0; j < kWords; ++j) {
-        const uint32_t t = lane + 32u * j, r = t / kWords, p = t % kWords;
+    for (uint32_t j = 0; j < COUNT; ++j) {
+        const uint32_t t = lane + 32u * j, r = t / COUNT, p = FIRST + t % COUNT;
         const uint32_t w = p < 12u ? p : p < 18u ? 33u + (p - 12u) : 50u + (p - 18u);
-        if (first + r < n) stage[r * kStride + p] = words[(size_t)(first + r) * kRecWords + w];
+        if (first + r < n) stage[r * STRIDE + p] = words[(size_t)(first + r) * kRecWords + w];
     }
     __syncwarp();
 }
@@ -501,7 +499,7 @@ __global__ void __launch_bounds__(kFeatBlock) features_kernel(const hydro_body* 
     __shared__ double stage[kFeatBlock / 32][32 * kFeatStride];
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const uint32_t first = blockIdx.x * kFeatBlock + 32u * wib;
-    stage_states<false>(bodies, first, n, stage[wib]);
+    stage_states<0, kFeatWords, kFeatStride>(bodies, first, n, stage[wib]);
     const uint32_t i = first + lane;
     if (i >= n) return;
     float o16[16];
@@ -580,43 +578,55 @@ cudaError_t launch_gate(const float* f, uint32_t n, const float* lo, const float
 
 // Features, gate and INSIDE test of a state in one pass over its record: three
 // launches of 16, 7 and 11 us for 65,536 states, of which the last read the
-// records again, 24 us as one (13 us for 16,384).
+// records again, 22.7 us as one (11.0 us for 16,384).  A wave lookup is a
+// chain of dependent loads and a state needs up to thirteen, so that two warps
+// share 32 states, one the features and the gate, one the INSIDE test (one
+// warp for both: 24 and 13 us).
 constexpr int kStateWords = kFeatWords + 6, kStateStride = kStateWords | 1;
 
-__global__ void __launch_bounds__(kFeatBlock) states_kernel(const hydro_body* __restrict__ bodies, uint32_t n,
-                                                            OceanDev o, GateParams g, float* __restrict__ f,
-                                                            uint8_t* __restrict__ mask)
+__global__ void __launch_bounds__(2 * kFeatBlock) states_kernel(const hydro_body* __restrict__ bodies, uint32_t n,
+                                                                OceanDev o, GateParams g, float* __restrict__ f,
+                                                                uint8_t* __restrict__ mask)
 {
     __shared__ double stage[kFeatBlock / 32][32 * kStateStride];
     __shared__ float Ps[256], ls[16], hs[16], ms[16];
+    __shared__ uint32_t inside[kFeatBlock / 32];   // a bit per state
     launch_dependents();
-    for (int k = threadIdx.x; k < 256; k += kFeatBlock) Ps[k] = g.P[k];
-    if (threadIdx.x < 16) {
-        ls[threadIdx.x] = g.lo[threadIdx.x];
-        hs[threadIdx.x] = g.hi[threadIdx.x];
-        ms[threadIdx.x] = g.mean[threadIdx.x];
-    }
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const uint32_t first = blockIdx.x * kFeatBlock + 32u * wib;
-    stage_states<true>(bodies, first, n, stage[wib]);
-    __syncthreads();
-    const uint32_t i = first + lane;
-    if (i >= n) return;
-    const double* sw = &stage[wib][lane * kStateStride];
-    float x[16];
-    state_features(sw, o, x);
-    float4* f4 = reinterpret_cast<float4*>(f + (size_t)i * 16);
+    const uint32_t lane = threadIdx.x & 31u, wib = (threadIdx.x % kFeatBlock) >> 5;
+    const uint32_t first = blockIdx.x * kFeatBlock + 32u * wib, i = first + lane;
+    double* sw = &stage[wib][lane * kStateStride];
+    bool in = false;
+    if (threadIdx.x < kFeatBlock) {
+        for (int k = threadIdx.x; k < 256; k += kFeatBlock) Ps[k] = g.P[k];
+        if (threadIdx.x < 16) {
+            ls[threadIdx.x] = g.lo[threadIdx.x];
+            hs[threadIdx.x] = g.hi[threadIdx.x];
+            ms[threadIdx.x] = g.mean[threadIdx.x];
+        }
+        stage_states<0, kFeatWords, kStateStride>(bodies, first, n, stage[wib]);
+        asm volatile("bar.sync 1, %0;" :: "n"(kFeatBlock) : "memory");   // the gate's parameters
+        if (i < n) {
+            float x[16];
+            state_features(sw, o, x);
+            float4* f4 = reinterpret_cast<float4*>(f + (size_t)i * 16);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) f4[k] = make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
-    bool in = gate_admits(x, Ps, ls, hs, ms, g.thresh);
-    if (in && g.inside) in = classify(o, sw + kFeatWords, sw + kFeatWords + 3) != HYDRO_INSIDE;
-    mask[i] = in ? 1 : 0;
+            for (int k = 0; k < 4; ++k) f4[k] = make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
+            in = gate_admits(x, Ps, ls, hs, ms, g.thresh);
+        }
+    } else if (g.inside) {
+        stage_states<kFeatWords, 6, kStateStride>(bodies, first, n, stage[wib]);
+        const bool t = i < n && classify(o, sw + kFeatWords, sw + kFeatWords + 3) == HYDRO_INSIDE;
+        const uint32_t bits = __ballot_sync(0xffffffffu, t);
+        if (lane == 0) inside[wib] = bits;
+    }
+    __syncthreads();
+    if (threadIdx.x < kFeatBlock && i < n) mask[i] = in && !(g.inside && (inside[wib] >> lane & 1u)) ? 1 : 0;
 }
 
 cudaError_t launch_states(const hydro_body* bodies, uint32_t n, OceanDev o, const GateParams& g, float* feats,
                           uint8_t* mask, cudaStream_t s)
 {
-    states_kernel<<<(n + kFeatBlock - 1) / kFeatBlock, kFeatBlock, 0, s>>>(bodies, n, o, g, feats, mask);
+    states_kernel<<<(n + kFeatBlock - 1) / kFeatBlock, 2 * kFeatBlock, 0, s>>>(bodies, n, o, g, feats, mask);
     return cudaGetLastError();
 }
 
