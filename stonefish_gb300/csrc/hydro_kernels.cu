@@ -1464,7 +1464,7 @@ static uint32_t body_cap(LaunchShape shape) { return 8u * (uint32_t)std::max(1, 
 // single body's call 43.3 -> 38.8 us, a hull among waves 67.7 -> 60.7, 1,000
 // spheres 46.8 -> 44.4).  The chunk kernel does not trigger early: the
 // finalisation's CTAs would all be placed on the SMs that run out of chunks
-// first (12,288 mixed bodies 268 us, without 259).  With events between the
+// first (4,096 mixed bodies 268 us, without 259).  With events between the
 // kernels they are launched as usual.
 static cudaError_t launch_chunks(const KParams& P, LaunchShape shape, int cut64, cudaStream_t s, cudaEvent_t* ev)
 {
