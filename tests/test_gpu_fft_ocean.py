@@ -27,6 +27,28 @@ def test_fft_ocean_matches_oracle(oracle, built_library, state, t):
     h.close()
 
 
+@pytest.mark.parametrize("passes", [2, 3, 9, 10])
+def test_fft_ocean_grid_sizes(oracle, built_library, passes):
+    """The smallest grids (four texels a row, one pair of columns a CTA), a
+    grid with more texels per CTA than threads in the columns, and the largest
+    one (rows too, and more shared memory than the default).  A channel shares
+    a complex field with its neighbour, whose rounding it carries: the error is
+    relative to the larger of the two."""
+    h = HydroContext(0)
+    p = fft_ocean_params(2.0)
+    p.passes = passes
+    fo = FftOcean(h, p)
+    for t in (0.4, 7.3):
+        fo.update(t)
+        gpu, ref = fo.read(), oracle.fft_ocean(p, t)
+        assert gpu.shape == ref.shape == (1 << passes, 1 << passes, 4)
+        for c in (0, 2):
+            scale = np.max(np.abs(ref[:, :, c:c + 2]))
+            assert np.max(np.abs(gpu[:, :, c:c + 2] - ref[:, :, c:c + 2])) < 1e-4 * scale, c
+    fo.close()
+    h.close()
+
+
 def test_hydrodynamics_on_the_fft_field(oracle, built_library):
     """Depths and a batched step read the field as the reference's
     ComputeWaveHeight does: channels 0 and 1 at grid sizes 893 m and 101 m."""
