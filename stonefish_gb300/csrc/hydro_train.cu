@@ -5,7 +5,7 @@
 // Step by step the layers' products, epilogues, transposes, column sums and
 // parameter updates are 36 launches of 3 to 15 us whose operands travel
 // through memory between them: 228 us at batch 4096, of which the tensor
-// cores need about 3; the fused step takes 42 us.  Here
+// cores need about 3; the fused step takes 40 us.  Here
 //   1. train_rows_kernel: 32 rows of the batch go through the four layers,
 //      the loss gradient and back to the first layer's pre-activations in
 //      one CTA.  No row needs another one, so the activations stay in shared
@@ -41,9 +41,12 @@ constexpr int kLdA = kH + 8;     // activation row stride in shared memory (an o
 // kernel issued an instruction in 23% of its cycles (two warps per scheduler
 // waiting on mma and ldmatrix results) and took 29 us; with sixteen 22 us.
 constexpr int kThreads = 512;
-constexpr int kStages = 3;
-constexpr int kStageBytes = 64 * kH * 2;   // 64 weight rows
-constexpr int kChunks = 22;      // weight chunks of the seven products
+// Chunks of 128 weight rows, the next one in flight: eleven CTA barriers for
+// the seven products.  With chunks of 64 and two in flight there were 22, and a
+// step took 1.4 us longer.
+constexpr int kStages = 2;
+constexpr int kStageBytes = 128 * kH * 2;   // 128 weight rows
+constexpr int kChunks = 11;      // weight chunks of the seven products
 constexpr size_t kRowsSmem = (size_t)kStages * kStageBytes + 2 * kRows * kLdA * 2 + (3 * kH + 64) * 4;
 
 __device__ __forceinline__ void cp16(void* dst, const void* src)
@@ -56,31 +59,31 @@ template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
 // Chunk i of the weights in the order the row kernel multiplies by them:
-// 64 rows of the layers' weights going forward, of their transposes going
-// back, 16-byte unit c of row r stored at unit c ^ (r % 8) so that ldmatrix
+// 128 rows of the layers' weights going forward, of their transposes going
+// back (64 or 256 where the layer is narrow), 16-byte unit c of row r stored at unit c ^ (r % 8) so that ldmatrix
 // reads eight rows without bank conflicts.  One commit group per chunk.
 __device__ __forceinline__ void load_weights(const RowsParams& P, unsigned char* smem, int i)
 {
     if (i < kChunks) {
         const bf16* src;
-        bool narrow = false;
-        if (i < 1) src = P.w16[0];
-        else if (i < 5) src = P.w16[1] + (i - 1) * 64 * kH;
-        else if (i < 9) src = P.w16[2] + (i - 5) * 64 * kH;
-        else if (i < 13) { src = P.w16[3] + (i - 9) * 64 * 64; narrow = true; }
-        else if (i < 14) src = P.wt16[3];
-        else if (i < 18) src = P.wt16[2] + (i - 14) * 64 * kH;
-        else src = P.wt16[1] + (i - 18) * 64 * kH;
+        int rows = 128;
+        if (i < 1) { src = P.w16[0]; rows = 64; }
+        else if (i < 3) src = P.w16[1] + (i - 1) * 128 * kH;
+        else if (i < 5) src = P.w16[2] + (i - 3) * 128 * kH;
+        else if (i < 6) { src = P.w16[3]; rows = 0; }   // 256 rows of 64
+        else if (i < 7) { src = P.wt16[3]; rows = 64; }
+        else if (i < 9) src = P.wt16[2] + (i - 7) * 128 * kH;
+        else src = P.wt16[1] + (i - 9) * 128 * kH;
         unsigned char* st = smem + (i % kStages) * kStageBytes;
-        if (narrow) {
+        if (rows == 0) {
 #pragma unroll
-            for (int j = 0; j < 64 * 8 / kThreads; ++j) {
+            for (int j = 0; j < 256 * 8 / kThreads; ++j) {
                 const int u = threadIdx.x + j * kThreads, r = u >> 3, c = u & 7;
                 cp16(st + r * 128 + ((c ^ (r & 7)) << 4), src + r * 64 + c * 8);
             }
         } else {
-#pragma unroll
-            for (int j = 0; j < 64 * 32 / kThreads; ++j) {
+#pragma unroll 4
+            for (int j = 0; j < rows * 32 / kThreads; ++j) {
                 const int u = threadIdx.x + j * kThreads, r = u >> 5, c = u & 31;
                 cp16(st + r * 512 + ((c ^ (r & 7)) << 4), src + r * kH + c * 8);
             }
@@ -116,20 +119,20 @@ __device__ __forceinline__ void product256(const RowsParams& P, unsigned char* s
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
+    const int rows = n_chunks == 1 ? 64 : 128;
 #pragma unroll 1
     for (int q = 0; q < n_chunks; ++q) {
         const int i = first + q;
-        cp_wait<1>();
+        cp_wait<0>();
         __syncthreads();   // chunk i is visible, and chunk i - 1's stage is free
-        load_weights(P, smem, i + 2);
-        if (q == 0 && out) store_rows(buf, out, out_cols);
+        load_weights(P, smem, i + 1);
         const unsigned char* st = smem + (i % kStages) * kStageBytes;
-#pragma unroll
-        for (int kk = 0; kk < 64; kk += 16) {
+#pragma unroll 8
+        for (int kk = 0; kk < rows; kk += 16) {
             uint32_t a[2][4], t[4];
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi)
-                ldsm_x4(a[mi], buf + (mi * 16 + (lane & 15)) * kLdA + q * 64 + kk + (lane >> 4) * 8);
+                ldsm_x4(a[mi], buf + (mi * 16 + (lane & 15)) * kLdA + q * 128 + kk + (lane >> 4) * 8);
             const int j = lane >> 3, r = kk + (lane & 7) + 8 * (j & 1), c = (wn >> 3) + (j >> 1);
             ldsm_x4_t(t, st + r * 512 + ((c ^ (r & 7)) << 4));
 #pragma unroll
@@ -138,6 +141,8 @@ __device__ __forceinline__ void product256(const RowsParams& P, unsigned char* s
                 mma_bf16(acc[mi][1], a[mi], t[2], t[3]);
             }
         }
+        // behind the first chunk's products: in front of them a step took 0.4 us longer
+        if (q == 0 && out) store_rows(buf, out, out_cols);
     }
 }
 
@@ -196,7 +201,6 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
     dependency_wait();
     launch_dependents();
     load_weights(P, smem, 0);
-    load_weights(P, smem, 1);
     if (tid < 256) {
         const int r = tid >> 3, c = tid & 7;
         *reinterpret_cast<uint4*>(buf0 + r * kLdA + c * 8) =
@@ -206,33 +210,29 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
     Tile d0, d1, d2;   // products, then SiLU derivatives, of the hidden layers
     product256(P, smem, buf0, 0, 1, nullptr, 0, d0);
     epilogue_silu(d0, bias, buf1);
-    product256(P, smem, buf1, 1, 4, P.x[0] + row0 * kH, kH, d1);
+    product256(P, smem, buf1, 1, 2, P.x[0] + row0 * kH, kH, d1);
     epilogue_silu(d1, bias + kH, buf0);
-    product256(P, smem, buf0, 5, 4, P.x[1] + row0 * kH, kH, d2);
+    product256(P, smem, buf0, 3, 2, P.x[1] + row0 * kH, kH, d2);
     epilogue_silu(d2, bias + 2 * kH, buf1);
     // output layer, N = 64: warp w's 16 x 8 tile; then the loss gradient
     {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         const int wm = (warp >> 3) * 16, wn = (warp & 7) * 8;
-#pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-            const int i = 9 + q;
-            cp_wait<1>();
-            __syncthreads();
-            load_weights(P, smem, i + 2);
-            if (q == 0) store_rows(buf1, P.x[2] + row0 * kH, kH);
-            const unsigned char* st = smem + (i % kStages) * kStageBytes;
-#pragma unroll
-            for (int kk = 0; kk < 64; kk += 32) {
-                uint32_t a[4], t[4];
-                const int r = kk + lane;   // four 8 x 8 matrices along k
-                ldsm_x4_t(t, st + r * 128 + (((wn >> 3) ^ (r & 7)) << 4));
-                ldsm_x4(a, buf1 + (wm + (lane & 15)) * kLdA + q * 64 + kk + (lane >> 4) * 8);
-                mma_bf16(acc, a, t[0], t[1]);
-                ldsm_x4(a, buf1 + (wm + (lane & 15)) * kLdA + q * 64 + kk + 16 + (lane >> 4) * 8);
-                mma_bf16(acc, a, t[2], t[3]);
-            }
+        cp_wait<0>();
+        __syncthreads();
+        load_weights(P, smem, 6);
+        const unsigned char* st = smem + (5 % kStages) * kStageBytes;
+#pragma unroll 2
+        for (int kk = 0; kk < kH; kk += 32) {
+            uint32_t a[4], t[4];
+            const int r = kk + lane;   // four 8 x 8 matrices along k
+            ldsm_x4_t(t, st + r * 128 + (((wn >> 3) ^ (r & 7)) << 4));
+            ldsm_x4(a, buf1 + (wm + (lane & 15)) * kLdA + kk + (lane >> 4) * 8);
+            mma_bf16(acc, a, t[0], t[1]);
+            ldsm_x4(a, buf1 + (wm + (lane & 15)) * kLdA + kk + 16 + (lane >> 4) * 8);
+            mma_bf16(acc, a, t[2], t[3]);
         }
+        store_rows(buf1, P.x[2] + row0 * kH, kH);
         const float scale = 1.f / (float)((size_t)P.batch * P.n_out);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -255,11 +255,11 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
         }
     }
     Tile acc;
-    product256(P, smem, buf0, 13, 1, P.dz[3] + row0 * 64, 64, acc);
+    product256(P, smem, buf0, 6, 1, P.dz[3] + row0 * 64, 64, acc);
     epilogue_grad(acc, d2, buf1);
-    product256(P, smem, buf1, 14, 4, P.dz[2] + row0 * kH, kH, acc);
+    product256(P, smem, buf1, 7, 2, P.dz[2] + row0 * kH, kH, acc);
     epilogue_grad(acc, d1, buf0);
-    product256(P, smem, buf0, 18, 4, P.dz[1] + row0 * kH, kH, acc);
+    product256(P, smem, buf0, 9, 2, P.dz[1] + row0 * kH, kH, acc);
     epilogue_grad(acc, d0, buf1);
     __syncthreads();
     store_rows(buf1, P.dz[0] + row0 * kH, kH);
@@ -486,7 +486,7 @@ __device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int 
 // A CTA updates 32 x 8 weights (the transposed copy leaves through shared
 // memory in 64-byte rows) or, the last four CTAs, one layer's biases.  Five
 // CTAs per SM take the 644 in one wave; with the four that unbounded registers
-// allow a second wave held 36 of them (10.8 us, now 7.8).  The parameters are
+// allow a second wave held 36 of them (10.8 us, now 6.4).  The parameters are
 // read before the wait: the step's row kernel has waited for the update that
 // wrote them, and this kernel is placed when the gradients' have all waited
 // for the row kernel.
