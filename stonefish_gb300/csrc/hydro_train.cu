@@ -486,10 +486,9 @@ __device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int 
 // A CTA updates 32 x 8 weights (the transposed copy leaves through shared
 // memory in 64-byte rows) or, the last four CTAs, one layer's biases.  Five
 // CTAs per SM take the 644 in one wave; with the four that unbounded registers
-// allow a second wave held 36 of them (10.8 us, now 6.4).  The parameters are
-// read before the wait: the step's row kernel has waited for the update that
-// wrote them, and this kernel is placed when the gradients' have all waited
-// for the row kernel.
+// allow a second wave held 36 of them (10.8 us, now 6.4).  The parameters too
+// are read behind the wait: the step before wrote them, and only a kernel that
+// has waited itself is promised to see what an earlier one of the chain wrote.
 __global__ void __launch_bounds__(256, 5) train_update_kernel(const UpdateParams P)
 {
     using namespace train;
@@ -504,8 +503,8 @@ __global__ void __launch_bounds__(256, 5) train_update_kernel(const UpdateParams
         if (b < count) {
             const int r = (b / tn) * 32 + (tid >> 3), c = (b % tn) * 8 + (tid & 7);
             const size_t i = (size_t)r * L.n + c, mn = (size_t)L.k * L.n;
-            const Moments o{L.w[i], L.mw[i], L.vw[i]};
             dependency_wait();
+            const Moments o{L.w[i], L.mw[i], L.vw[i]};
             const float g = ordered_sum(L.part + i, mn, L.splits);
             L.gw[i] = g;
             const bf16 h = __float2bfloat16(adamw(P, o, L.w, L.mw, L.vw, i, g, P.wd));
