@@ -869,8 +869,8 @@ typedef struct hydro_nn_net {
  * hydro_nn_transpose, hydro_nn_colsum and hydro_nn_adamw, so the trained
  * weights are the same bits as calling those one by one; a step costs no
  * round trip through the caller, and a 64-256-256-256-64 network runs it in
- * three fused launches.  w, b, their moments and bf16 copies, gw, gb and
- * *loss are the results; z, x, dz and xt are scratch. */
+ * three fused launches.  gw, gb, z, x, dz and xt hold the last step's values
+ * afterwards, as far as they don't share memory. */
 hydro_status hydro_nn_train(hydro_ctx* ctx, const hydro_nn_net* net, const void* X, const float* T,
                             int64_t n_rows, const int64_t* rows, const float* lr, int32_t n_steps,
                             int32_t step0, float beta1, float beta2, float eps, float weight_decay,

@@ -10,7 +10,8 @@
 //      the loss gradient and back to the first layer's pre-activations in
 //      one CTA.  No row needs another one, so the activations stay in shared
 //      memory and the FP32 pre-activations in registers; only the BF16
-//      layer inputs and gradients that the weight gradients need are written.
+//      layer inputs and gradients that the weight gradients need are written
+//      (in a call's last step the pre-activations too).
 //   2. train_grads_kernel: every layer's weight-gradient product (split
 //      along the batch), bias column sums and the loss, side by side.  The
 //      transposed operand is formed by ldmatrix.trans, not by a transpose
@@ -147,8 +148,10 @@ __device__ __forceinline__ void product256(const RowsParams& P, unsigned char* s
 }
 
 // Hidden layer: z = acc + bias, SiLU(z) into `y`; acc keeps SiLU'(z), all
-// that the way back needs of z (one sigmoid serves both).
-__device__ __forceinline__ void epilogue_silu(Tile& acc, const float* bias, bf16* y)
+// that the way back needs of z (one sigmoid serves both).  KEEP: z to memory
+// as well.
+template <bool KEEP>
+__device__ __forceinline__ void epilogue_silu(Tile& acc, const float* bias, bf16* y, float* z)
 {
     const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) * 16;
 #pragma unroll
@@ -161,6 +164,7 @@ __device__ __forceinline__ void epilogue_silu(Tile& acc, const float* bias, bf16
             for (int h = 0; h < 2; ++h) {
                 const int r = mi * 16 + (lane >> 2) + 8 * h;
                 const float z0 = acc[mi][ni][2 * h] + b.x, z1 = acc[mi][ni][2 * h + 1] + b.y;
+                if (KEEP) *reinterpret_cast<float2*>(z + (size_t)r * kH + c) = make_float2(z0, z1);
                 const float s0 = sigmoidf_(z0), s1 = sigmoidf_(z1);
                 *reinterpret_cast<__nv_bfloat162*>(y + r * kLdA + c) =
                     __nv_bfloat162(__float2bfloat16(z0 * s0), __float2bfloat16(z1 * s1));
@@ -189,6 +193,8 @@ __device__ __forceinline__ void epilogue_grad(const Tile& acc, const Tile& d, bf
 
 }  // namespace train
 
+// KEEP: the call's last step, which leaves every pre-activation in memory.
+template <bool KEEP>
 __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const RowsParams P)
 {
     using namespace train;
@@ -209,11 +215,11 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
     for (int i = tid; i < 3 * kH + 64; i += kThreads) bias[i] = P.bias[i >> 8][i & 255];
     Tile d0, d1, d2;   // products, then SiLU derivatives, of the hidden layers
     product256(P, smem, buf0, 0, 1, nullptr, 0, d0);
-    epilogue_silu(d0, bias, buf1);
+    epilogue_silu<KEEP>(d0, bias, buf1, P.z[0] + row0 * kH);
     product256(P, smem, buf1, 1, 2, P.x[0] + row0 * kH, kH, d1);
-    epilogue_silu(d1, bias + kH, buf0);
+    epilogue_silu<KEEP>(d1, bias + kH, buf0, P.z[1] + row0 * kH);
     product256(P, smem, buf0, 3, 2, P.x[1] + row0 * kH, kH, d2);
-    epilogue_silu(d2, bias + 2 * kH, buf1);
+    epilogue_silu<KEEP>(d2, bias + 2 * kH, buf1, P.z[2] + row0 * kH);
     // output layer, N = 64: warp w's 16 x 8 tile; then the loss gradient
     {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -241,12 +247,12 @@ __global__ void __launch_bounds__(train::kThreads, 1) train_rows_kernel(const Ro
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 g[e] = 0.f;
+                const float z = acc[2 * h + e] + bias[3 * kH + c + e];
+                if (KEEP || c + e < P.n_out) P.z[3][(row0 + r) * 64 + c + e] = z;   // for the loss
                 if (c + e < P.n_out) {
-                    const float z = acc[2 * h + e] + bias[3 * kH + c + e];
                     float tv = P.target[(row0 + r) * P.n_out + c + e];
                     if (P.tmean) tv = (tv - P.tmean[c + e]) * P.tistd[c + e];
                     const float d = z - tv;
-                    P.z3[(row0 + r) * 64 + c + e] = z;   // for the loss
                     g[e] = 2.f * d * scale;
                 }
             }
@@ -526,10 +532,11 @@ __global__ void __launch_bounds__(256, 5) train_update_kernel(const UpdateParams
     }
 }
 
-cudaError_t launch_train_step(const RowsParams& R, const GradsParams& G, const UpdateParams& U, cudaStream_t s)
+cudaError_t launch_train_step(const RowsParams& R, const GradsParams& G, const UpdateParams& U, bool keep,
+                              cudaStream_t s)
 {
-    cudaError_t e = cudaFuncSetAttribute(train_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)train::kRowsSmem);
+    const void* rows = keep ? (const void*)train_rows_kernel<true> : (const void*)train_rows_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train::kRowsSmem);
     if (e != cudaSuccess) return e;
     int grads = 256, updates = 4;   // loss blocks; bias blocks
     for (const GradLayer& L : G.layer) grads += (L.k / 64) * (L.n / 64) * L.splits + (L.n / 32) * L.slabs;
@@ -538,9 +545,7 @@ cudaError_t launch_train_step(const RowsParams& R, const GradsParams& G, const U
     void* ar[] = {const_cast<RowsParams*>(&R)};
     void* ag[] = {const_cast<GradsParams*>(&G)};
     void* au[] = {const_cast<UpdateParams*>(&U)};
-    if ((e = launch_chained((const void*)train_rows_kernel, R.batch / train::kRows, train::kThreads, train::kRowsSmem, s,
-                            ar)))
-        return e;
+    if ((e = launch_chained(rows, R.batch / train::kRows, train::kThreads, train::kRowsSmem, s, ar))) return e;
     if ((e = launch_chained((const void*)train_grads_kernel, grads, train::kGradThreads, 0, s, ag))) return e;
     return launch_chained((const void*)train_update_kernel, updates, 256, 0, s, au);
 }

@@ -8,8 +8,9 @@
 namespace sfh {
 
 // Rows forward and back: x0 [batch][64] inputs, target [batch][n_out]; the
-// BF16 layer inputs x and gradients dz are outputs, z3 [batch][64] receives
-// the network's outputs (first n_out columns).
+// BF16 layer inputs x and gradients dz are outputs; z[3] [batch][64] receives
+// the network's outputs (first n_out columns) or, where a step keeps them,
+// every z [batch][n_l] its layer's pre-activations.
 struct RowsParams {
     const __nv_bfloat16* x0;
     const float* target;
@@ -20,7 +21,7 @@ struct RowsParams {
     const float* bias[4];
     __nv_bfloat16* x[3];
     __nv_bfloat16* dz[4];
-    float* z3;
+    float* z[4];
     int batch;
     int n_out;
 };
@@ -64,6 +65,8 @@ struct UpdateParams {
     float lr, b1, b2, eps, wd, bc1, bc2;
 };
 
-cudaError_t launch_train_step(const RowsParams& R, const GradsParams& G, const UpdateParams& U, cudaStream_t s);
+// keep: leave the pre-activations in R.z
+cudaError_t launch_train_step(const RowsParams& R, const GradsParams& G, const UpdateParams& U, bool keep,
+                              cudaStream_t s);
 
 }  // namespace sfh

@@ -105,3 +105,31 @@ def test_fused_step_for_other_targets(hctx, n_out, normalise):
     _native(hctx, sur, X, T, _net(sur, n_out, stats))
     _same(sur, ref)
     assert np.isclose(float(sur.loss_d), float(ref.loss_d), rtol=1e-12)
+
+
+@pytest.mark.parametrize("n_out,shared_xt", [(6, False), (5, True)])
+def test_buffers_hold_the_last_step(hctx, n_out, shared_xt):
+    """After a call z (every column), x, dz and xt hold what the last step's
+    single entry points leave there, also with one xt for all layers."""
+    ref, X, T, stats = _problem(hctx, 6, n_out)
+    _step_by_step(hctx, ref, X, T, n_out, stats)
+    sur, X, T, stats = _problem(hctx, 6, n_out)
+    bufs = sur._bufs()
+    for group in bufs.values():
+        for t in group:
+            t.fill_(7.0)
+    net = _net(sur, n_out, stats)
+    if shared_xt:
+        for l in range(4):
+            net.xt[l] = bufs["xt"][1].data_ptr()
+    _native(hctx, sur, X, T, net)
+    _same(sur, ref)
+    want = ref._bufs()
+    for key in ("z", "x", "dz"):
+        for l, (a, b) in enumerate(zip(bufs[key], want[key])):
+            assert torch.equal(a, b), (key, l)
+    if shared_xt:   # the first layer's input comes last
+        assert torch.equal(bufs["xt"][1].view(-1)[:64 * BATCH], want["xt"][0].view(-1))
+    else:
+        for l in range(4):
+            assert torch.equal(bufs["xt"][l], want["xt"][l]), l
