@@ -972,7 +972,9 @@ typedef struct hydro_nn_predict_net {
 /* Gated prediction of n states (device pointers).  n_nets 1 or 2; the gate of
  * hydro_nn_gate, with gate_inside that of hydro_nn_gate_inside; two networks
  * give their mean and the gate of hydro_nn_ensemble at tau (infinity: off).
- * audit_stride > 0 samples as hydro_nn_audit_pick does.  Work buffers:
+ * audit_stride > 0 samples as hydro_nn_audit_pick does.  The scales are
+ * those of hydro_nn_ensemble and hydro_nn_audit_error (positive where one of
+ * the two is in use).  Work buffers:
  * features [n][16], mask [n], counts [(n + 255) / 256], packed [n], pos [n],
  * rows [n], n_packed [1], exact [n]; features, z and out 16-byte aligned.
  * Every field is read at the call. */

@@ -2449,9 +2449,11 @@ extern "C" hydro_status hydro_nn_predict(hydro_ctx* ctx, hydro_batch* batch, con
         return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: missing argument");
     const hydro_nn_predictor& q = *p;
     if (q.n == 0 || q.n != batch->n_bodies || q.n >= kAuditedRow || !q.lo || !q.hi || !q.mean || !q.precision || !q.err || !q.features || !q.mask ||
-        !q.counts || !q.packed || !q.pos || !q.rows || !q.n_packed || !q.exact || !q.out || !(q.force_scale > 0.0) ||
-        !(q.torque_scale > 0.0) || (q.audit_stride && (!d_audit_err || audit_phase >= q.audit_stride)))
+        !q.counts || !q.packed || !q.pos || !q.rows || !q.n_packed || !q.exact || !q.out || (q.audit_stride && (!d_audit_err || audit_phase >= q.audit_stride)))
         return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: bad predictor");
+    // the scales measure two networks' disagreement and the audit's errors
+    if ((q.n_nets > 1 || q.audit_stride) && !(q.force_scale > 0.0 && q.torque_scale > 0.0))
+        return fail(ctx, HYDRO_ERR_INVALID_ARG, "nn predict: scales must be positive");
     uintptr_t align = reinterpret_cast<uintptr_t>(q.features) | reinterpret_cast<uintptr_t>(q.out);
     for (int k = 0; k < q.n_nets; ++k) {
         const hydro_nn_predict_net& N = q.net[k];

@@ -1,0 +1,66 @@
+"""GatedPredictor (hydro_nn_predict): what a caller reads beside the outputs,
+and how one state's prediction stands to the others of its call."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from stonefish_gb300 import scenarios  # noqa: E402
+from stonefish_gb300 import surrogate as S  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+class Scene:
+    """A hull, a wave field, states and untrained networks normalised on
+    them, with the gates wide open."""
+
+    def __init__(self, n, nets=1, faces=3000, gravity=None):
+        from stonefish_gb300.hydro import HydroContext
+        self.h = HydroContext()
+        self.mid = self.h.upload_mesh(*S.hull_mesh(faces))
+        self.h.set_wave_grid(scenarios.wave_grid(n=256, n_waves=16, seed=5))
+        self.ocean, self.st, self.n = S.wave_ocean(), scenarios.settings(), n
+        if gravity is not None:
+            self.ocean.gravity = gravity
+        self.bodies = S.sample_states(np.random.default_rng(n), n, extent=25.6)
+        self.bodies["mesh"] = self.mid
+        self.d_b = torch.from_numpy(self.bodies.view(np.uint8).copy()).cuda()
+        rng = np.random.default_rng(1)
+        feats = torch.from_numpy(rng.normal(size=(4096, S.N_FEAT)).astype(np.float32)).cuda()
+        targ = torch.from_numpy((rng.normal(size=(4096, S.N_OUT)) * 500.0).astype(np.float32)).cuda()
+        self.nets = [S.Surrogate(self.h, batch=256, seed=k) for k in range(nets)]
+        for net in self.nets:
+            net.fit_normalisation(feats, targ)
+            net.gate["lo"].fill_(-1e30), net.gate["hi"].fill_(1e30)
+            net.gate["thr"] = 1e30
+
+    def predictor(self, **kw):
+        return S.GatedPredictor(self.nets[0], self.h, self.mid, self.n, self.ocean, self.st,
+                                second=self.nets[1] if len(self.nets) > 1 else None, **kw)
+
+
+@pytest.fixture
+def scene(built_library):
+    open_ = []
+
+    def make(*a, **kw):
+        open_.append(Scene(*a, **kw))
+        return open_[-1]
+    yield make
+    for s in open_:
+        s.h.close()
+
+
+def test_one_network_needs_no_scales(scene):
+    """Without a second network and without the audit nothing is measured
+    against the hull's force scale, which is zero without gravity."""
+    s = scene(300, gravity=0.0)
+    gp = s.predictor()
+    assert gp.fs == 0.0
+    got = gp.predict(s.d_b).cpu().numpy()
+    z = torch.zeros((300, 16), device="cuda")
+    feats = gp.bufs["feats"][:300].contiguous()
+    s.nets[0].infer_tc(feats, z, gp.tcw)
+    assert np.array_equal(got, z[:, :6].cpu().numpy()) and gp.rejected() == 0
+    gp.close()
