@@ -161,9 +161,7 @@ class Rollout:
             self._ck(self.lib.hydro_rigid_step(self.h.ctx, _ptr(self.states), _ptr(self.bodies), _ptr(self.io),
                                                None, self.n, self.dt, self.gravity, s))
             return self.batch.last_launches() + 1
-        # whole chunks: a trajectory then does not depend on how many other
-        # hulls the gate sends to the exact step
-        out = self.pred.predict(self.bodies, split_chunks=False)
+        out = self.pred.predict(self.bodies)
         self._ck(self.lib.hydro_rigid_step(self.h.ctx, _ptr(self.states), _ptr(self.bodies), None, _ptr(out),
                                            self.n, self.dt, self.gravity, s))
         return self.pred.launches + 1

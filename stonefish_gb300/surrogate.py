@@ -582,11 +582,14 @@ class GatedPredictor:
     def _ck(self, st):
         _check(self.lib, self.h.ctx, st)
 
-    def predict(self, d_bodies: torch.Tensor, split_chunks: bool = True) -> torch.Tensor:
+    def predict(self, d_bodies: torch.Tensor, split_chunks: bool = False) -> torch.Tensor:
         """d_bodies: bytes of n hydro_body on the device, or in page-locked
         host memory, which the kernels then read in place (mesh ids are
         ignored: the exact slots use this predictor's mesh).  Returns out
-        [n,6] (device)."""
+        [n,6] (device).  ``split_chunks``: while few states take the exact
+        step, its chunks are cut into smaller ones, which is faster, but the
+        order of a state's FP32 sums then depends on how many others of the
+        call take that step too ("tcgen05" only)."""
         s = self.s
         st = s._s()
         n, b = self.n, self.bufs

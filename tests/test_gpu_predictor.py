@@ -64,3 +64,25 @@ def test_one_network_needs_no_scales(scene):
     s.nets[0].infer_tc(feats, z, gp.tcw)
     assert np.array_equal(got, z[:, :6].cpu().numpy()) and gp.rejected() == 0
     gp.close()
+
+
+@pytest.mark.parametrize("n", [600, 6000])
+def test_prediction_is_a_states_own(scene, n):
+    """A state's output is the same bits however many others of its call take
+    the exact step: here the gate's depth limit lets few or most through."""
+    s = scene(n)
+    gp = s.predictor()
+    gp.predict(s.d_b)
+    depth = gp.bufs["feats"][:n, 0].clone()
+    outs = []
+    for q in (0.99, 0.9, 0.2):
+        s.nets[0].gate["hi"][0] = float(torch.quantile(depth, q))
+        outs.append((gp.predict(s.d_b).clone(), gp.pos.clone() >= 0))
+        assert 0 < gp.rejected() < n
+    few = outs[0][1]
+    for out, exact in outs[1:]:
+        assert bool((exact | ~few).all()) and int(exact.sum()) > int(few.sum())
+        assert torch.equal(out[few], outs[0][0][few])
+        both = ~exact
+        assert torch.equal(out[both], outs[0][0][both])
+    gp.close()
