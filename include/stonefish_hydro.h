@@ -1003,6 +1003,7 @@ typedef struct hydro_nn_predictor {
     uint32_t* n_packed;
     hydro_wrench* exact;
     float* out;
+    int32_t* audit_idx;
 } hydro_nn_predictor;
 
 /* out [n][6] = the networks' body-frame wrench for the states the gates admit
@@ -1012,7 +1013,8 @@ typedef struct hydro_nn_predictor {
  * in six launches (fourteen with two networks and the audit).  `batch` holds
  * n bodies of one mesh.  With split_chunks the exact step's chunks are split
  * into smaller ones while few states take it, which changes the order of its
- * FP32 sums (not their accuracy) with the number of such states.  audit_err: one float per sample.
+ * FP32 sums (not their accuracy) with the number of such states.
+ * audit_err: one float per sample; audit_idx (optional): its row or -1.
  * *launches (optional) receives the kernels launched. */
 hydro_status hydro_nn_predict(hydro_ctx* ctx, hydro_batch* batch, const hydro_nn_predictor* p,
                               const hydro_body* d_states, const hydro_ocean* ocean, const hydro_settings* settings,

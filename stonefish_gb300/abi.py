@@ -155,7 +155,7 @@ class NnPredictor(C.Structure):
                 ("force_scale", C.c_double), ("torque_scale", C.c_double), ("lo", C.c_void_p), ("hi", C.c_void_p), ("mean", C.c_void_p),
                 ("precision", C.c_void_p), ("net", NnPredictNet * 2), ("err", C.c_void_p), ("features", C.c_void_p),
                 ("mask", C.c_void_p), ("counts", C.c_void_p), ("packed", C.c_void_p), ("pos", C.c_void_p),
-                ("rows", C.c_void_p), ("n_packed", C.c_void_p), ("exact", C.c_void_p), ("out", C.c_void_p)]
+                ("rows", C.c_void_p), ("n_packed", C.c_void_p), ("exact", C.c_void_p), ("out", C.c_void_p), ("audit_idx", C.c_void_p)]
 
 
 class TuneResult(C.Structure):

@@ -2484,7 +2484,7 @@ extern "C" hydro_status hydro_nn_predict(hydro_ctx* ctx, hydro_batch* batch, con
     if (e == cudaSuccess) e = launch_mlp_nets(q.features, q.n, nets, q.n_nets, q.err, s);
     if (e == cudaSuccess)
         e = launch_combine(q.net[0].z, q.n_nets > 1 ? q.net[1].z : nullptr, q.n, inv_fs, inv_ts, q.tau, q.audit_stride,
-                           audit_phase, d_audit_err, q.mask, q.counts, q.out, s);
+                           audit_phase, d_audit_err, q.audit_idx, q.mask, q.counts, q.out, s);
     if (e == cudaSuccess)
         e = launch_predict_step(P, d_states, q.mask, q.n, q.counts, q.packed, q.pos, q.rows, q.n_packed, shape,
                                 ctx->cfg.cut_precision == HYDRO_CUT_FP64, s);

@@ -227,12 +227,13 @@ struct GateParams {
 cudaError_t launch_states(const hydro_body* bodies, uint32_t n, OceanDev o, const GateParams& g, float* feats,
                           uint8_t* mask, cudaStream_t s);
 // Mean of the networks' outputs (into z0), disagreement gate, audit sample,
-// outputs of the admitted states, rejects per block of kCombineBlock states.
+// outputs of the admitted states, rejects per block of kCombineBlock states;
+// audit_idx (may be null): the sample's rows, as audit_pick_kernel gives them.
 // mask: 1 admitted, 0 rejected, 2 audited.
 constexpr int kCombineBlock = 256;
 cudaError_t launch_combine(float* z0, const float* z1, uint32_t n, float inv_fs, float inv_ts, float tau,
-                           uint32_t audit_stride, uint32_t audit_phase, float* audit_err, uint8_t* mask,
-                           uint32_t* counts, float* out, cudaStream_t s);
+                           uint32_t audit_stride, uint32_t audit_phase, float* audit_err, int32_t* audit_idx,
+                           uint8_t* mask, uint32_t* counts, float* out, cudaStream_t s);
 // The exact step for the rejected states: packed in index order (with the
 // per-body preparation), chunk kernel, finalisation with the merge of P.
 cudaError_t launch_predict_step(const KParams& P, const hydro_body* states, uint8_t* mask, uint32_t n,

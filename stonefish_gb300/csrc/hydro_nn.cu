@@ -808,8 +808,9 @@ cudaError_t launch_ensemble(float* za, const float* zb, int ld, uint32_t n, floa
 // outputs (merge_kernel's copy) and route_count_kernel's counts.
 __global__ void __launch_bounds__(kCombineBlock)
 combine_kernel(float* __restrict__ z0, const float* __restrict__ z1, uint32_t n, float inv_fs, float inv_ts, float tau,
-               uint32_t audit_stride, uint32_t audit_phase, float* __restrict__ audit_err, uint8_t* __restrict__ mask,
-               uint32_t* __restrict__ counts, float* __restrict__ out)
+               uint32_t audit_stride, uint32_t audit_phase, float* __restrict__ audit_err,
+               int32_t* __restrict__ audit_idx, uint8_t* __restrict__ mask, uint32_t* __restrict__ counts,
+               float* __restrict__ out)
 {
     const uint32_t i = blockIdx.x * kCombineBlock + threadIdx.x;
     bool reject = false;
@@ -817,7 +818,10 @@ combine_kernel(float* __restrict__ z0, const float* __restrict__ z1, uint32_t n,
     dependency_wait();
     if (i == 0 && audit_stride) {   // the last sample may lie past the last state
         const uint32_t last = (n - 1) / audit_stride;
-        if ((uint64_t)last * audit_stride + audit_phase >= n) audit_err[last] = -1.f;
+        if ((uint64_t)last * audit_stride + audit_phase >= n) {
+            audit_err[last] = -1.f;
+            if (audit_idx) audit_idx[last] = -1;
+        }
     }
     if (i < n) {
         float a[6];
@@ -847,8 +851,10 @@ combine_kernel(float* __restrict__ z0, const float* __restrict__ z1, uint32_t n,
         }
         uint8_t m = reject ? 0 : 1;
         if (audit_stride && i >= audit_phase && (i - audit_phase) % audit_stride == 0) {
+            const uint32_t j = (i - audit_phase) / audit_stride;
             if (!reject) m = 2;   // audited: exact as well; its error is written by the finalisation
-            else audit_err[(i - audit_phase) / audit_stride] = -1.f;
+            else audit_err[j] = -1.f;
+            if (audit_idx) audit_idx[j] = reject ? -1 : (int32_t)i;
             reject = true;
         }
         mask[i] = m;
@@ -864,10 +870,11 @@ combine_kernel(float* __restrict__ z0, const float* __restrict__ z1, uint32_t n,
 }
 
 cudaError_t launch_combine(float* z0, const float* z1, uint32_t n, float inv_fs, float inv_ts, float tau,
-                           uint32_t audit_stride, uint32_t audit_phase, float* audit_err, uint8_t* mask,
-                           uint32_t* counts, float* out, cudaStream_t s)
+                           uint32_t audit_stride, uint32_t audit_phase, float* audit_err, int32_t* audit_idx,
+                           uint8_t* mask, uint32_t* counts, float* out, cudaStream_t s)
 {
-    void* args[] = {&z0, &z1, &n, &inv_fs, &inv_ts, &tau, &audit_stride, &audit_phase, &audit_err, &mask, &counts, &out};
+    void* args[] = {&z0,        &z1,        &n,    &inv_fs, &inv_ts, &tau, &audit_stride, &audit_phase,
+                    &audit_err, &audit_idx, &mask, &counts, &out};
     return launch_chained((const void*)combine_kernel, (n + kCombineBlock - 1) / kCombineBlock, kCombineBlock, 0, s, args);
 }
 

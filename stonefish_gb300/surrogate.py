@@ -577,6 +577,7 @@ class GatedPredictor:
         for k in ("counts", "packed", "pos", "rows", "n_packed", "out"):
             setattr(p, k, getattr(self, k).data_ptr())
         p.exact = self.exact_io.data_ptr()
+        p.audit_idx = self.audit_idx.data_ptr() if self.audit_k else None
         return p
 
     def _ck(self, st):

@@ -86,3 +86,23 @@ def test_prediction_is_a_states_own(scene, n):
         both = ~exact
         assert torch.equal(out[both], outs[0][0][both])
     gp.close()
+
+
+@pytest.mark.parametrize("n,stride", [(1, 4), (63, 64), (500, 64), (4097, 1024)])
+def test_audit_rows_are_recorded(scene, n, stride):
+    """audit_idx holds the call's sample: a row for each audited state, -1 for
+    one the gate sent to the exact step anyway or a slot past the last state."""
+    s = scene(n)
+    gp = s.predictor(audit_stride=stride)
+    gp.predict(s.d_b)
+    s.nets[0].gate["hi"][0] = float(torch.quantile(gp.bufs["feats"][:n, 0], 0.6))
+    feats, hi = gp.bufs["feats"][:n].clone(), s.nets[0].gate["hi"]
+    admitted = (feats[:, 0] <= hi[0]).cpu().numpy()
+    for call in range(1, 4):
+        gp.audit_idx.fill_(-7)
+        gp.predict(s.d_b)
+        rows = call % stride + stride * np.arange(gp.audit_k)
+        want = np.where((rows < n) & admitted[np.minimum(rows, n - 1)], rows, -1)
+        assert np.array_equal(gp.audit_idx.cpu().numpy(), want)
+        assert np.array_equal(gp.audit_err[call].cpu().numpy() >= 0, want >= 0)
+    gp.close()
