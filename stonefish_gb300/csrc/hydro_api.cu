@@ -455,6 +455,15 @@ hydro_status batch_params(hydro_batch* b, const hydro_body* d_bodies, const hydr
     return HYDRO_OK;
 }
 
+// Kernel timing events (hydro_batch_profile) of a step on s: outside stream
+// capture only.
+cudaEvent_t* step_events(hydro_batch* b, cudaStream_t s)
+{
+    if (!b->prof_ev[0]) return nullptr;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone ? b->prof_ev : nullptr;
+}
+
 hydro_status batch_launch(hydro_batch* b, const hydro_body* d_bodies, const hydro_ocean* ocean,
                           const hydro_settings* settings, hydro_wrench* d_io, cudaStream_t s,
                           int op, const uint32_t* d_count = nullptr, hydro_aero_wrench* d_aero = nullptr,
@@ -467,12 +476,7 @@ hydro_status batch_launch(hydro_batch* b, const hydro_body* d_bodies, const hydr
     if (st != HYDRO_OK) return st;
     const int cut64 = ctx->cfg.cut_precision == HYDRO_CUT_FP64;
     uint32_t launches = 0;
-    // kernel timing events (hydro_batch_profile) outside stream capture only
-    cudaEvent_t* ev = nullptr;
-    if (b->prof_ev[0]) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) ev = b->prof_ev;
-    }
+    cudaEvent_t* ev = step_events(b, s);
     cudaError_t e = launch_step(P, shape, cut64, s, &launches, ev);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "wrench step launch");
     b->last_launches = launches;
@@ -2480,6 +2484,7 @@ extern "C" hydro_status hydro_nn_predict(hydro_ctx* ctx, hydro_batch* batch, con
         nets[k] = PredictNet{N.fmean, N.fistd, N.image, {N.bias[0], N.bias[1], N.bias[2], N.bias[3]}, N.z};
     }
     const GateParams g{q.lo, q.hi, q.mean, q.precision, q.threshold, q.gate_inside};
+    cudaEvent_t* ev = step_events(batch, s);
     cudaError_t e = launch_states(d_states, q.n, P.ocean, g, q.features, q.mask, s);
     if (e == cudaSuccess) e = launch_mlp_nets(q.features, q.n, nets, q.n_nets, q.err, s);
     if (e == cudaSuccess)
@@ -2487,7 +2492,11 @@ extern "C" hydro_status hydro_nn_predict(hydro_ctx* ctx, hydro_batch* batch, con
                            audit_phase, d_audit_err, q.audit_idx, q.mask, q.counts, q.out, s);
     if (e == cudaSuccess)
         e = launch_predict_step(P, d_states, q.mask, q.n, q.counts, q.packed, q.pos, q.rows, q.n_packed, shape,
-                                ctx->cfg.cut_precision == HYDRO_CUT_FP64, s);
+                                ctx->cfg.cut_precision == HYDRO_CUT_FP64, s, ev);
+    if (e == cudaSuccess) {
+        batch->last_launches = 3u;   // of the exact step: packing with preparation, chunks, finalisation
+        if (ev) batch->prof_recorded = true;
+    }
     if (launches) *launches = 6u;
     NN_RET(e, "nn predict");
 }

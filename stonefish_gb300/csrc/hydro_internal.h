@@ -238,7 +238,8 @@ cudaError_t launch_combine(float* z0, const float* z1, uint32_t n, float inv_fs,
 // per-body preparation), chunk kernel, finalisation with the merge of P.
 cudaError_t launch_predict_step(const KParams& P, const hydro_body* states, uint8_t* mask, uint32_t n,
                                 const uint32_t* counts, hydro_body* packed, int32_t* pos, uint32_t* rows,
-                                uint32_t* n_packed, LaunchShape shape, int cut64, cudaStream_t s);
+                                uint32_t* n_packed, LaunchShape shape, int cut64, cudaStream_t s,
+                                cudaEvent_t* ev);
 cudaError_t launch_mlp_tc(const float* feats, uint32_t n, const float* fmean, const float* fistd,
                           const void* wimg, const float* b0, const float* b1, const float* b2, const float* b3,
                           float* out, unsigned* err, cudaStream_t s);

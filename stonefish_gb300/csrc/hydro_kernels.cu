@@ -1506,14 +1506,17 @@ cudaError_t launch_step(const KParams& P, LaunchShape shape, int cut64, cudaStre
 
 cudaError_t launch_predict_step(const KParams& P, const hydro_body* states, uint8_t* mask, uint32_t n,
                                 const uint32_t* counts, hydro_body* packed, int32_t* pos, uint32_t* rows,
-                                uint32_t* n_packed, LaunchShape shape, int cut64, cudaStream_t s)
+                                uint32_t* n_packed, LaunchShape shape, int cut64, cudaStream_t s,
+                                cudaEvent_t* ev)
 {
     const uint32_t nb = (n + kCombineBlock - 1) / kCombineBlock;
     void* args[] = {const_cast<KParams*>(&P), &states, &mask, &n, &counts, const_cast<uint32_t*>(&nb), &packed, &pos,
                     &rows, &n_packed};
-    const cudaError_t e = launch_chained((const void*)predict_pack_kernel, nb, kCombineBlock, 0, s, args);
-    if (e != cudaSuccess) return e;
-    return launch_chunks(P, shape, cut64, s, nullptr);
+    cudaError_t e;
+    if (ev && (e = cudaEventRecord(ev[0], s))) return e;
+    if ((e = launch_chained((const void*)predict_pack_kernel, nb, kCombineBlock, 0, s, args, !ev))) return e;
+    if (ev && (e = cudaEventRecord(ev[1], s))) return e;
+    return launch_chunks(P, shape, cut64, s, ev);
 }
 
 // ------------------------------------------------------------- compounds

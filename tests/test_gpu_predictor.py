@@ -106,3 +106,28 @@ def test_audit_rows_are_recorded(scene, n, stride):
         assert np.array_equal(gp.audit_idx.cpu().numpy(), want)
         assert np.array_equal(gp.audit_err[call].cpu().numpy() >= 0, want >= 0)
     gp.close()
+
+
+def test_exact_step_is_profiled_and_counted(scene):
+    """hydro_batch_profile and hydro_batch_last_launches of the predictor's
+    batch see the exact step of a prediction, whose outputs stay the same."""
+    s = scene(3000)
+    gp = s.predictor()
+    gp.predict(s.d_b)
+    s.nets[0].gate["hi"][0] = float(torch.quantile(gp.bufs["feats"][:3000, 0], 0.7))
+    plain = gp.predict(s.d_b).clone()
+    assert gp.batch.last_launches() == 3 and gp.rejected() > 0
+    gp.batch.profile(True)
+    assert torch.equal(gp.predict(s.d_b), plain)
+    ms = gp.batch.kernel_ms()
+    assert all(0.0 < ms[k] < 50.0 for k in ("prep", "chunk", "finalize")), ms
+    g = torch.cuda.CUDAGraph()          # no events while a stream captures
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(g, stream=side):
+        gp.predict(s.d_b)
+    gp.out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(gp.out, plain)
+    gp.close()
