@@ -276,6 +276,14 @@ struct WaveTaps {
     float alpha, beta;
 };
 
+// Whether no index of a lookup is N, in one comparison; their OR would pass
+// only where N is a power of two, and send a fifth of all points of other
+// grids through the general form as well.
+__host__ __device__ __forceinline__ bool texels_in_grid(uint32_t i0, uint32_t i1, uint32_t j0, uint32_t j1, uint32_t N)
+{
+    return max(max(i0, i1), max(j0, j1)) < N;
+}
+
 // OpenGLRealOcean::ComputeInterpolatedWaveData (OpenGLRealOcean.cpp:282-319),
 // texel-centred periodic bilinear; the linear texel index wraps modulo N*N
 // where the reference would read texel N of a row.  False, and offsets that
@@ -296,7 +304,7 @@ __device__ __forceinline__ bool wave_taps(const OceanDev& o, float x, float y, W
     t.l1 = j0 * N + i1;
     t.l2 = j1 * N + i0;
     t.l3 = j1 * N + i1;
-    return fabsf(x) < 0x1p21f && fabsf(y) < 0x1p21f && (i0 | i1 | j0 | j1) < N;
+    return fabsf(x) < 0x1p21f && fabsf(y) < 0x1p21f && texels_in_grid(i0, i1, j0, j1, N);
 }
 
 __device__ __forceinline__ void wave_taps_wide(const OceanDev& o, float x, float y, WaveTaps& t)
