@@ -421,7 +421,7 @@ static_assert(offsetof(hydro_body, T_CG) == 0 && offsetof(hydro_body, v) == 33 *
               "feature words of hydro_body");
 
 // The features of a state from its 18 staged words.
-__device__ __forceinline__ void state_features(const double* sw, const OceanDev& o, float (&o16)[16])
+__device__ __forceinline__ void state_features(const double* sw, const OceanDev& o, float* o16)
 {
     double R[9];
 #pragma unroll
@@ -502,10 +502,7 @@ __global__ void __launch_bounds__(kFeatBlock) features_kernel(const hydro_body* 
     stage_states<0, kFeatWords, kFeatStride>(bodies, first, n, stage[wib]);
     const uint32_t i = first + lane;
     if (i >= n) return;
-    float o16[16];
-    state_features(&stage[wib][lane * kFeatStride], o, o16);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) f[(size_t)i * 16 + k] = o16[k];
+    state_features(&stage[wib][lane * kFeatStride], o, f + (size_t)i * 16);
 }
 
 cudaError_t launch_features(const hydro_body* bodies, uint32_t n, OceanDev o, float* f, cudaStream_t s)
