@@ -68,7 +68,7 @@ __device__ void fluid_velocity64(const OceanDev& o, const double* p, double* fv)
         } else if (c.type == HYDRO_CURRENT_JET) {
             add_jet_velocity(c, p, fv);
         } else if (c.type == HYDRO_CURRENT_PIPE) {
-            add_pipe_velocity(c, p, fv);
+            add_pipe_velocity<true>(c, p, fv);
         }
     }
 }

@@ -446,6 +446,11 @@ __device__ __forceinline__ void bcross(const double* a, const double* b, double*
 // pipe profile's power as exp(gamma log).  200 bodies of up to 12,288 faces
 // between a jet and a pipe, FP64 cuts: chunk kernel 306 us with every
 // current evaluated at every face, 210 us.
+// A pipe's last two are kept from velocities that leave in FP64 (WIDE: cables):
+// exp(gamma log y) is off by up to gamma |log y| units of 2^-53 where pow is
+// off by one, which a face's velocity, rounded to FP32, does not show (the
+// same bits on three fleets of 200 bodies, whose calls take 320 us with pow
+// and 280 us without).
 __device__ __forceinline__ double dot3d(const double* a, const double* b) { return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0])); }
 
 // |p x dir|^2 of the axis distance
@@ -473,6 +478,7 @@ __device__ inline void add_jet_velocity(const hydro_current& c, const double* p,
 }
 
 // Pipe::GetVelocityAtPoint (Pipe.cpp:57-79), FP64, added to fv
+template <bool WIDE>
 __device__ inline void add_pipe_velocity(const hydro_current& c, const double* p, double* fv)
 {
     const double pp[3] = {p[0] - c.point[0], p[1] - c.point[1], p[2] - c.point[2]};
@@ -481,12 +487,16 @@ __device__ inline void add_pipe_velocity(const hydro_current& c, const double* p
     const double d2 = axis_distance2(pp, c.dir);
     const double r = c.radius + (c.radius2 - c.radius) * t / c.length;
     if (r <= 0.0 || d2 >= r * r) return;
-    const double ir = 1.0 / r;
-    const double y = fma(-sqrt(d2), ir, 1.0);
-    // the profile's exponent is a small positive number (1/7 for turbulent
-    // flow); any other goes through pow
-    const double f = c.gamma > 0.0 && c.gamma < 64.0 ? exp(c.gamma * log(fmax(y, 0.0))) : pow(y, c.gamma);
-    const double s = c.radius * ir * c.speed * f;
+    double s;
+    if (WIDE) {
+        s = c.radius / r * c.speed * pow(1.0 - sqrt(d2) / r, c.gamma);
+    } else {
+        const double ir = 1.0 / r;
+        const double y = fmax(fma(-sqrt(d2), ir, 1.0), 0.0);
+        // the profile's exponent is a small positive number (1/7 for turbulent
+        // flow); any other goes through pow
+        s = c.radius * ir * c.speed * (c.gamma > 0.0 && c.gamma <= 1.0 ? exp(c.gamma * log(y)) : pow(y, c.gamma));
+    }
     for (int k = 0; k < 3; ++k) fv[k] = fma(c.dir[k], s, fv[k]);
 }
 
@@ -526,7 +536,7 @@ __device__ __forceinline__ v3 field_velocity(const OceanDev& o, v3 pt, float ox,
             for (int k = 0; k < 3; ++k) fv[k] += c.vel[k];
         } else if ((hit >> i) & 1u) {
             if (c.type == HYDRO_CURRENT_JET) add_jet_velocity(c, p, fv);
-            else if (c.type == HYDRO_CURRENT_PIPE) add_pipe_velocity(c, p, fv);
+            else if (c.type == HYDRO_CURRENT_PIPE) add_pipe_velocity<false>(c, p, fv);
         }
     }
     return mk((float)fv[0], (float)fv[1], (float)fv[2]);
