@@ -16,10 +16,12 @@
 // Bound: GB300 retires about two FP64 lanes per clock per SM, so the time is
 // the number of FP64 operations.  A segment wholly on one side of the surface
 // by more than the radius, which is most of them, needs neither its angle nor
-// a share of its volume, and the angle's cosine and sine are quotients of its
-// sides instead of cos(atan()) and sin(atan()).  300 cables of 100 to 400
-// nodes: 147 us with one warp per cable going through its segments 32 at
-// a time with those functions, 49 us now (63 before the items were spread).
+// a share of its volume.  What is left runs the reference's operations one by
+// one: the angle's cosine and sine as quotients of the sides are no faster
+// (51.5 and 53.7 us) and a tenth less accurate where a segment crosses the
+// surface; fused and regrouped drag products save 2 us.  300 cables of 100 to
+// 400 nodes: 147 us with one warp per cable going through its segments 32 at
+// a time, all with the angle, 54 us now.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -95,8 +97,8 @@ __device__ void segment(const OceanDev& o, SettingsDev st, const hydro_cable& cb
     if (f2 < -rf && rf > 0.f) return;                         // out of the water
     const double d1 = (double)f1, d2 = (double)f2;
     const double sv[3] = {xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]};
-    const double h2 = fma(sv[1], sv[1], sv[0] * sv[0]);
-    const double L = sqrt(fma(sv[2], sv[2], h2));
+    const double h2 = sv[0] * sv[0] + sv[1] * sv[1];
+    const double L = sqrt(h2 + sv[2] * sv[2]);
     double V = 0.0;
     bool full = f1 > rf && rf > 0.f;
     if (full) {
@@ -104,18 +106,7 @@ __device__ void segment(const OceanDev& o, SettingsDev st, const hydro_cable& cb
     } else {
         const double dz = d2 - d1;
         const double dxy = h2 > kEps ? sqrt(h2) : 0.0;        // btVector3::safeNorm
-        // cos and sin of alpha = atan(dz / dxy), dz >= 0
-        const double hyp = sqrt(dz * dz + dxy * dxy);
-        double ca, sa;
-        if (hyp > 0.0 && hyp < 1e150) {
-            const double inv = 1.0 / hyp;
-            ca = dxy * inv;
-            sa = dz * inv;
-        } else {                                              // no length, overflow or NaN
-            const double alpha = atan(dz / dxy);
-            ca = cos(alpha);
-            sa = sin(alpha);
-        }
+        const double alpha = atan(dz / dxy), ca = cos(alpha), sa = sin(alpha);
         const double margin = fuzzy_zero(dxy) ? 0.0 : r * ca;
         if (d2 < -margin) {
             return;                                           // out of the water
@@ -160,13 +151,13 @@ __device__ void segment(const OceanDev& o, SettingsDev st, const hydro_cable& cb
         }
         for (int k = 0; k < 3; ++k) rv[k] = fma(va[k] + vb[k], 0.5, -rv[k]);
         const double Cd = 0.5;
-        const double f1v = fabs(fma(sv[2], rv[2], fma(sv[1], rv[1], sv[0] * rv[0])));
+        const double f1v = fabs(sv[0] * rv[0] + sv[1] * rv[1] + sv[2] * rv[2]);
         // a full segment's share is its volume over itself, one (not so for an infinite volume)
         const double share = full && V < 1e300 ? 1.0 : V / (kPi * r * r * L);
-        const double rl = sqrt(fma(rv[2], rv[2], fma(rv[1], rv[1], rv[0] * rv[0])));
-        const double a = share * (r * L);
-        const double q = (f1v - 1.0) * a * (o.density * Cd) * rl;   // -(1 - f1) share rho / 2 Cd (2 r L) |v|
-        const double Sf = -(2.0 * kPi) * a;
+        const double rl = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
+        const double S = 2.0 * r * L;
+        const double q = -(1.0 - f1v) * share * 0.5 * o.density * Cd * S * rl;
+        const double Sf = -(share * ((2.0 * kPi) * r * L));
         for (int k = 0; k < 3; ++k) {
             out9[3 + k] = q * rv[k];
             out9[6 + k] = Sf * rv[k];
