@@ -884,8 +884,12 @@ hydro_status hydro_wave_grid_set(hydro_ctx* ctx, const float* data, uint32_t siz
     if (ctx->wave_d) cudaFree(ctx->wave_d);
     ctx->wave_d = nullptr;
     const size_t bytes = (size_t)size * size * channels * sizeof(float);
-    CK(ctx, cudaMalloc(&ctx->wave_d, bytes));
+    // the lookup wraps a linear index once, which leaves a grid of one texel at
+    // its second where both fractions round up to one: a copy of the first
+    const size_t spare = size == 1 ? bytes : 0;
+    CK(ctx, cudaMalloc(&ctx->wave_d, bytes + spare));
     CK(ctx, cudaMemcpy(ctx->wave_d, data, bytes, cudaMemcpyHostToDevice));
+    if (spare) CK(ctx, cudaMemcpy(ctx->wave_d + channels, data, bytes, cudaMemcpyHostToDevice));
     ctx->wave_n = size;
     ctx->wave_channels = channels;
     ctx->wave_layers = n_layers;

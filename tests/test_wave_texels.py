@@ -98,3 +98,23 @@ def _positions(h, ocean, lo, hi):
     h._ck(h.lib.hydro_nn_gate_inside(h.ctx, S._ptr(d_b), len(lo), C.byref(ocean), S._ptr(mask), None))
     torch.cuda.synchronize()
     return mask.cpu().numpy() == 0
+
+
+@pytest.mark.gpu
+def test_grid_of_one_texel(oracle, built_library):
+    """One texel of two channels: both fractions round up to one beside the
+    wrap, and the index wraps back to the texel."""
+    from stonefish_gb300.hydro import HydroContext
+    waves = {"data": np.array([[[0.75, -0.5]]], dtype=np.float32), "layers": [(0, 4.0), (1, 8.0)]}
+    ocean = scenarios.flat_ocean()
+    ocean.waves = 1
+    u = np.concatenate([[0.5], np.nextafter(np.float32(0.5), np.float32([0, 1])), [-0.5, 0.0, 3.25, 1e9]]).astype(np.float32)
+    x, y = np.meshgrid(np.concatenate([u * 4, u * 8]), np.concatenate([u * 4, u * 8]))
+    pts = np.stack([x.ravel(), y.ravel(), np.ones(x.size)], 1).astype(np.float32)
+    h = HydroContext(0)
+    try:
+        h.set_wave_grid(waves)
+        ref = np.array([oracle.depth(ocean, waves, *map(float, p)) for p in pts], dtype=np.float32)
+        assert np.array_equal(h.depth(ocean, pts), ref)
+    finally:
+        h.close()
