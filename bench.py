@@ -14,6 +14,9 @@ with the inputs resident in HBM (``value``), and through the host-buffer C ABI
 call with the host<->device copies inside the timed region (``e2e``).  The
 mesh data (~0.5 GB) is larger than L2, so no flush is needed between steps.
 
+The measurement is printed as one JSON line; the full report (every error
+figure, the surrogate's and the rollout's sections) goes to ``--report``.
+
 ``--impl reference`` times the reference's own routine on the host cores
 on the same workload: its hydrodynamics functions compiled from its sources
 (oracle/_ref) where they were built on this machine, else the oracle's REF32
@@ -865,8 +868,43 @@ def run_reference(args, rank: int):
             "e2e": {"value": value, "unit": unit, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
 
 
+# Sections of the report: the printed line has their numbers and short words
+# only, and these of their own sections.
+SECTIONS = {"roofline": (), "issue_roofline": (), "kernel_config": (), "error_vs_fp64": (), "cpu_baseline": (),
+            "surrogate": (("exact_fp32_gpu", "value"), ("error", "wrench_p99"), ("e2e", "value")),
+            "rollout": (("exact", "env_steps_per_s"), ("surrogate", "env_steps_per_s"))}
+LINE_CHARS = 3000   # a reader of the output's last few thousand characters gets the whole line
+
+
+def short_line(res: dict) -> str:
+    """The measurement as one JSON line of at most LINE_CHARS characters: the
+    contract's keys whole, the report's sections by their numbers."""
+    def number(v):
+        return float(f"{v:.6g}") if isinstance(v, float) else v
+
+    line = {}
+    for key, val in res.items():
+        if key not in SECTIONS or not isinstance(val, dict):
+            line[key] = val
+            continue
+        line[key] = {k: number(v) for k, v in val.items()
+                     if isinstance(v, (int, float)) or (isinstance(v, str) and len(v) <= 24)}
+        for a, b in SECTIONS[key]:
+            if isinstance(val.get(a), dict) and b in val[a]:
+                line[key][f"{a}_{b}"] = number(val[a][b])
+    if isinstance(line.get("e2e"), dict):
+        line["e2e"] = {k: v for k, v in line["e2e"].items() if k != "transfer"}
+    # further sections go before the contract's keys would
+    for key in ("kernel_config", "error_vs_fp64", "issue_roofline", "rollout", "surrogate", "roofline"):
+        if len(json.dumps(line)) > LINE_CHARS:
+            line.pop(key, None)
+    return json.dumps(line)
+
+
 def main():
     ap = argparse.ArgumentParser()
+    ap.add_argument("--report", default="bench_report.json",
+                    help="file for the full report (the printed line has its main figures); empty: none")
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=2000)
     ap.add_argument("--warmup", type=int, default=20)
@@ -915,8 +953,18 @@ def main():
         res = run_gpu(args, rank, world, local_rank, dist)
         if dist is not None:
             dist.destroy_process_group()
-    if res is not None:
+    if res is None:
+        return
+    if args.impl == "reference":
         print(json.dumps(res), flush=True)
+        return
+    if args.report:
+        try:
+            with open(args.report, "w") as f:
+                json.dump(res, f, indent=1)
+        except OSError as e:
+            print(f"no report: {e}", file=sys.stderr)
+    print(short_line(res), flush=True)
 
 
 if __name__ == "__main__":
