@@ -131,3 +131,95 @@ def test_exact_step_is_profiled_and_counted(scene):
     torch.cuda.synchronize()
     assert torch.equal(gp.out, plain)
     gp.close()
+
+
+@pytest.mark.parametrize("n,stride", [(257, 7), (3000, 64), (5000, 0)])
+def test_disagreement_gate_and_whole_chunks(scene, n, stride):
+    """Two networks with a threshold in the middle of their disagreements: the
+    gate alone rejects states, some of them audit rows; masks, slots and, with
+    whole chunks, every output are the bits of the single entry points'
+    chain.  The same call with chunks split stays within 2e-6 of the scales."""
+    import ctypes as C
+    s = scene(n, nets=2)
+    h, lib, ctx, P = s.h, s.h.lib, s.h.ctx, S._ptr
+    wide = s.predictor(tau=1e30)
+    wide.predict(s.d_b)
+    f = wide.bufs["feats"][:n].clone()
+    za, zb = torch.zeros((n, 16), device="cuda"), torch.zeros((n, 16), device="cuda")
+    s.nets[0].infer_tc(f, za, wide.tcw)
+    s.nets[1].infer_tc(f, zb, wide.tcw2)
+    d = torch.maximum((za - zb)[:, :3].double().norm(dim=1) / wide.fs, (za - zb)[:, 3:6].double().norm(dim=1) / wide.ts)
+    tau = float(torch.quantile(d, 0.9))
+    wide.close()
+    gp = s.predictor(tau=tau, audit_stride=stride)
+    got = gp.predict(s.d_b).clone()
+    mask = torch.ones(n, dtype=torch.uint8, device="cuda")
+    h._ck(lib.hydro_nn_ensemble(ctx, P(za), P(zb), 16, n, gp.fs, gp.ts, tau, P(mask), None))
+    gate = mask.clone()
+    idx = torch.zeros(max(gp.audit_k, 1), dtype=torch.int32, device="cuda")
+    if stride:
+        h._ck(lib.hydro_nn_audit_pick(ctx, P(mask), n, stride, 0, gp.audit_k, P(idx), None))
+        rows = torch.arange(0, n, stride, device="cuda")
+        assert 0 < int((gate[rows] == 0).sum()) < rows.numel()   # rejected audit rows, and admitted ones
+    rejected = int((gate == 0).sum())
+    assert 0.05 * n < rejected < 0.15 * n
+    clear = (d - tau).abs() > 1e-5 * tau
+    assert torch.equal((gate == 0)[clear], (d > tau)[clear])
+    cnt = torch.zeros((n + 255) // 256, dtype=torch.int32, device="cuda")
+    packed, pos = torch.zeros_like(s.d_b), torch.zeros(n, dtype=torch.int32, device="cuda")
+    npk, io = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(n * 168, dtype=torch.uint8, device="cuda")
+    h._ck(lib.hydro_nn_route(ctx, P(s.d_b), P(mask), n, P(cnt), P(packed), P(pos), P(npk), P(io), None))
+    gp.batch.compute_device_prefix(packed.data_ptr(), npk.data_ptr(), s.ocean, s.st, io.data_ptr())
+    out = torch.zeros((n, 6), device="cuda")
+    h._ck(lib.hydro_nn_merge(ctx, P(s.d_b), P(za), 16, P(pos), P(io), n, P(out), None))
+    torch.cuda.synchronize()
+    assert torch.equal(gp.bufs["mask"][:n], mask) and torch.equal(gp.pos, pos)
+    assert torch.equal(got, out)
+    if stride:
+        err = torch.zeros(gp.audit_k, device="cuda")
+        h._ck(lib.hydro_nn_audit_error(ctx, P(s.d_b), P(za), 16, P(pos), P(io), P(idx), gp.audit_k, gp.fs, gp.ts, P(err),
+                                       None))
+        assert torch.equal(gp.audit_idx, idx) and torch.allclose(gp.audit_err[0], err, rtol=1e-6, atol=1e-9)
+    p = gp._predictor(True)             # chunks split where few states are exact
+    launches = C.c_uint32()
+    h._ck(lib.hydro_nn_predict(ctx, gp.batch.b, C.byref(p), P(s.d_b), C.byref(s.ocean), C.byref(s.st), 0,
+                               P(gp.audit_err[1]) if stride else None, C.byref(launches), s.nets[0]._s()))
+    torch.cuda.synchronize()
+    ex = pos >= 0
+    scale = torch.tensor([gp.fs] * 3 + [gp.ts] * 3, device="cuda")
+    assert launches.value == 6 and torch.equal(gp.out[~ex], out[~ex])
+    if int(ex.sum()) <= 100:          # fewer chunks than half the CTAs
+        assert not torch.equal(gp.out[ex], out[ex])
+    assert float(((gp.out - out)[ex].abs() / scale).max()) <= 2e-6
+    gp.close()
+
+
+def test_refused_predictors(scene):
+    """Arguments that hydro_nn_predict refuses, before anything is launched."""
+    import ctypes as C
+
+    from stonefish_gb300 import abi
+    s = scene(300, nets=2)
+    gp = s.predictor(audit_stride=16)
+    other = s.h.upload_mesh(*S.hull_mesh(2000))
+    mixed = s.h.batch(np.array([s.mid, other] * 150, dtype=np.uint32))
+    short = s.h.batch(np.full(299, s.mid, dtype=np.uint32))
+    err, st = gp.audit_err[0], s.nets[0]._s()
+
+    def status(batch=gp.batch, phase=0, err=err, ocean=s.ocean, **changes):
+        p = gp._predictor(False)
+        for k, v in changes.items():
+            setattr(p, k, v)
+        return s.h.lib.hydro_nn_predict(s.h.ctx, batch.b, C.byref(p), S._ptr(s.d_b), C.byref(ocean), C.byref(s.st), phase,
+                                        S._ptr(err) if err is not None else None, None, st)
+
+    assert status() == 0
+    gp.out.fill_(5.0)
+    refused = [status(batch=mixed), status(batch=short), status(phase=16), status(err=None), status(n=0), status(n_nets=0),
+               status(n_nets=3), status(force_scale=0.0), status(torque_scale=-1.0), status(force_scale=float("nan")),
+               status(features=gp.bufs["feats"].data_ptr() + 4), status(out=gp.out.data_ptr() + 8), status(mask=None),
+               status(rows=None)]
+    assert refused == [abi.HYDRO_ERR_INVALID_ARG] * len(refused)
+    torch.cuda.synchronize()
+    assert bool((gp.out == 5.0).all())
+    gp.close(), mixed.close(), short.close()
