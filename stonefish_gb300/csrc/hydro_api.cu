@@ -1560,7 +1560,6 @@ hydro_status hydro_fft_ocean_read(hydro_fft_ocean* o, float* out)
 }
 
 // ----------------------------------------------------------------- cables
-// Segment scratch (9 doubles per node) followed by one error word.
 hydro_status hydro_cable_forces_device(hydro_ctx* ctx, const hydro_cable* d_cables, uint32_t n_cables,
                                        const double* d_x, const double* d_v, uint32_t n_nodes_total,
                                        const hydro_ocean* ocean, const hydro_settings* settings,

@@ -122,7 +122,7 @@ struct FieldBound {
     float length;
     float reach;
     float slope;
-    float size;          // |point|_1 + reach
+    float size;          // |point|_1 + |reach| and a pipe's |length|
     float scale;         // 1e-5 (1 + |dir|_1)
 };
 

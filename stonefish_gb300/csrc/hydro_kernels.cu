@@ -549,15 +549,6 @@ __device__ __forceinline__ void prefetch_lines(const void* p, size_t bytes, int 
         asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
 }
 
-// Appends the chunks of a body that runs a face loop (`n` of them, 0 for a
-// body without one or a lane without a body) to the launch's list of active
-// chunks, each into the region of its claim class (its tile count), so that
-// the producers never claim the chunks of bodies outside the water or
-// switched off, and claim the largest chunks first.  Called by all 32 lanes
-// of a warp.  A body's chunks are full (the work list's tiles per chunk)
-// except its last: the warp's full chunks take one run of their class (one
-// atomic, runs prefix-summed with shuffles, descriptors formed from the
-// body's first chunk), the last chunks one atomic per class present.
 // Lists a body's chunks cut into parts of `part` tiles (f parts per chunk at
 // most; part q of chunk c keeps its sums in slot c * f + q).  Called by all 32
 // lanes of a warp for a batch with one mesh, where every body has the same
@@ -595,6 +586,15 @@ __device__ __forceinline__ void list_parts(const KParams& P, uint32_t body, cons
     }
 }
 
+// Appends the chunks of a body that runs a face loop (`n` of them, 0 for a
+// body without one or a lane without a body) to the launch's list of active
+// chunks, each into the region of its claim class (its tile count), so that
+// the producers never claim the chunks of bodies outside the water or
+// switched off, and claim the largest chunks first.  Called by all 32 lanes
+// of a warp.  A body's chunks are full (the work list's tiles per chunk)
+// except its last: the warp's full chunks take one run of their class (one
+// atomic, runs prefix-summed with shuffles, descriptors formed from the
+// body's first chunk), the last chunks one atomic per class present.
 __device__ __forceinline__ void list_chunks(const KParams& P, uint32_t body, const BodyInfo& bi, uint32_t n)
 {
     const unsigned lane = threadIdx.x & 31u;

@@ -1,7 +1,7 @@
 // hydro_mlp_tc.cu -- fused inference of the wrench surrogate on the 5th-
 // generation tensor cores: a CTA takes blocks of 128 states through all four
-// layers (16 -> 256 -> 256 -> 256 -> 16) with the activations kept in shared
-// memory and the accumulators in tensor memory.
+// layers (16 -> 256 -> 256 -> 256 -> 16) with the activations and the
+// accumulators in tensor memory.
 //
 //   * persistent: a CTA per SM loops over pairs of 128-state blocks, both in
 //     flight: while one block's epilogue runs, the tensor pipe works for the
