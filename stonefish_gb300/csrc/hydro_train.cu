@@ -5,7 +5,7 @@
 // Step by step the layers' products, epilogues, transposes, column sums and
 // parameter updates are 36 launches of 3 to 15 us whose operands travel
 // through memory between them: 228 us at batch 4096, of which the tensor
-// cores need about 3; the fused step takes 40 us.  Here
+// cores need about 3; the fused step takes 41 us.  Here
 //   1. train_rows_kernel: 32 rows of the batch go through the four layers,
 //      the loss gradient and back to the first layer's pre-activations in
 //      one CTA.  No row needs another one, so the activations stay in shared
@@ -492,7 +492,7 @@ __device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int 
 // A CTA updates 32 x 8 weights (the transposed copy leaves through shared
 // memory in 64-byte rows) or, the last four CTAs, one layer's biases.  Five
 // CTAs per SM take the 644 in one wave; with the four that unbounded registers
-// allow a second wave held 36 of them (10.8 us, now 6.4).  The parameters too
+// allow a second wave held 36 of them (10.8 us, now 6.5).  The parameters too
 // are read behind the wait: the step before wrote them, and only a kernel that
 // has waited itself is promised to see what an earlier one of the chain wrote.
 __global__ void __launch_bounds__(256, 5) train_update_kernel(const UpdateParams P)
