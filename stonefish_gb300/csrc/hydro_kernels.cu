@@ -140,7 +140,7 @@ __device__ void finalize_surface(const OceanDev& o, int buoyancy, int damping,
 {
     const double V6 = S[Q_V6];
     if (buoyancy && V6 > (double)1e-9f) {
-        w.Vsub = V6 * (1.0 / 6.0);
+        w.Vsub = V6 / 6.0;
         if (o.waves) {
             const double k = o.density * o.gravity;
             set3(w.Fb, S[Q_FB] * k, S[Q_FB + 1] * k, S[Q_FB + 2] * k);
